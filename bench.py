@@ -33,13 +33,15 @@ METRIC = "J+K build ms & ERI quartets/s, mixed vs FP64 at <=1e-6 Eh; HF gradient
 MIXED_CUTOFF = 1e-6
 THRS = 1e-12
 # dgf_class_time.kernel: 0 thread-per-quartet, 1 cooperative team, 2 warp teams, 4 warp-per-quartet
-KERNEL_KIND = {0: "thread", 1: "team", 2: "team", 4: "warp", 6: "warp"}
+KERNEL_KIND = {0: "thread", 1: "team", 2: "team", 4: "warp", 6: "warp", 8: "row", 10: "pack"}
 
 
 def kernel_name(kind, la, lb, lc, ld, precision):
     """Template name of a profiled class kernel (kind as dgf_class_time.kernel;
     the warp kernel's last argument says whether its transforms run on the
     FP64 tensor cores)."""
+    if kind in (8, 10):
+        return f"jk_{KERNEL_KIND[kind]}_kernel<{la},{lb},{lc},{ld}>"
     t = "double" if precision == 64 else "float"
     mma = {4: ",false", 6: ",true"}.get(kind, "")
     return f"jk_{KERNEL_KIND[kind]}_kernel<{la},{lb},{lc},{ld},{t}{mma}>"

@@ -23,7 +23,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
-         "-ccbin", "g++", "-I", INCLUDE, "-I", CSRC]
+         "-ccbin", "g++", "--compress-mode=size", "-I", INCLUDE, "-I", CSRC]
 
 
 def _deps(path, seen=None):
@@ -78,7 +78,7 @@ def _generated_units():
     gen = os.path.join(BUILD, "gen")
     os.makedirs(gen, exist_ok=True)
     units = []
-    for kind, header, macro, n, parts in (("jk", None, None, NUM_PAIR_CLASS, 3),
+    for kind, header, macro, n, parts in (("jk", None, None, NUM_PAIR_CLASS, 5),
                                           ("grad", "dgf_grad_kernel.cuh", "DGF_GRAD_CLASS", NUM_GRAD_CLASS, 0)):
         for x in range(n):
             for y in range(x + 1):
@@ -89,6 +89,12 @@ def _generated_units():
                     elif part == 0:  # cooperative, warp-team and warp-per-quartet kernels
                         path = os.path.join(gen, f"dgf_{kind}_{x}_{y}_0.cu")
                         text = f'#include "dgf_jk_inst_team.cuh"\n\nDGF_JK_TEAM_CLASS({x}, {y})\n'
+                    elif part == 3:  # row kernels
+                        path = os.path.join(gen, f"dgf_{kind}_{x}_{y}_3.cu")
+                        text = f'#include "dgf_jk_inst_row.cuh"\n\nDGF_JK_ROW_CLASS({x}, {y})\n'
+                    elif part == 4:  # pack kernels
+                        path = os.path.join(gen, f"dgf_{kind}_{x}_{y}_4.cu")
+                        text = f'#include "dgf_jk_inst_pack.cuh"\n\nDGF_JK_PACK_CLASS({x}, {y})\n'
                     else:  # thread kernels, FP64 (1) or FP32 (2)
                         path = os.path.join(gen, f"dgf_{kind}_{x}_{y}_{part}.cu")
                         text = f'#include "dgf_jk_inst_thread.cuh"\n\nDGF_JK_THREAD_CLASS({x}, {y}, {part})\n'

@@ -15,6 +15,7 @@
 #include "dgf_ctx.h"
 #include "dgf_sph.h"
 #include "dgf_md.cuh"
+#include "dgf_pack.h"
 
 using namespace dgf;
 
@@ -113,6 +114,45 @@ void boys_table_host(std::vector<double> &out) {
   }
 }
 
+// Fine table of the row kernels: on each interval the Chebyshev interpolant of
+// F_M at kFineDeg + 1 nodes as a polynomial in x in [-1, 1], then e^-mid.
+// The interpolation error, at most (1/16)^8 / (2^7 8!) = 4.5e-17 times
+// F_{M+8}/F_M < 1, is below the rounding of F_M.
+void boys_fine_host(std::vector<double> &out) {
+  const long double pi = 3.14159265358979323846264338327950288L;
+  out.assign((size_t)(kFineMaxM + 1) * kFineDoubles, 0.0);
+  constexpr int n = kFineDeg + 1;
+  long double tk[n * n] = {}, cs[n * n];  // monomial coefficients of T_j; cos(pi j (k + 1/2) / n)
+  tk[0] = 1.0L;
+  tk[n + 1] = 1.0L;
+  for (int j = 2; j < n; ++j)
+    for (int k = 0; k < n; ++k) tk[j * n + k] = (k > 0 ? 2.0L * tk[(j - 1) * n + k - 1] : 0.0L) - tk[(j - 2) * n + k];
+  for (int j = 0; j < n; ++j)
+    for (int k = 0; k < n; ++k) cs[j * n + k] = cosl(pi * j * (k + 0.5L) / n);
+  const long double h = 1.0L / kFinePerUnit;
+  for (int i = 0; i < kFineNint; ++i) {
+    const long double mid = (i + 0.5L) * h;
+    long double f[kFineMaxM + 1][n];
+    for (int k = 0; k < n; ++k) {  // F_max by its series, the lower orders by downward recursion
+      const long double t = mid + 0.5L * h * cs[n + k], et = expl(-t);
+      f[kFineMaxM][k] = boys_series(kFineMaxM, t);
+      for (int m = kFineMaxM - 1; m >= 0; --m) f[m][k] = (2.0L * t * f[m + 1][k] + et) / (2 * m + 1);
+    }
+    for (int M = 0; M <= kFineMaxM; ++M) {
+      long double pw[n] = {};
+      for (int j = 0; j < n; ++j) {
+        long double c = 0.0L;
+        for (int k = 0; k < n; ++k) c += f[M][k] * cs[j * n + k];
+        c *= (j == 0 ? 1.0L : 2.0L) / n;
+        for (int k = 0; k < n; ++k) pw[k] += c * tk[j * n + k];
+      }
+      double *row = &out[(size_t)M * kFineDoubles + (size_t)i * kFineStride];
+      for (int k = 0; k < n; ++k) row[k] = (double)pw[k];
+      row[n] = (double)expl(-mid);
+    }
+  }
+}
+
 // Cartesian -> real spherical coefficients with Dalton's conventions (SPHCO1,
 // DALTON/abacus/her1pro.F:4697-4770, MORDER=1 so m = -l..l, MINTEG=2 so the
 // functions are normalised given Cartesians carrying the x^l norm), from the
@@ -131,15 +171,26 @@ void sph_table_host(std::vector<double> &out) {
 
 static void free_ctx(dgf_ctx *c) {
   if (!c) return;
+  free_ctx(c->prim);
   int prev = 0;
   cudaGetDevice(&prev);
   cudaSetDevice(c->device);
   void *ptrs[] = {c->d_pairs, c->d_pp,     c->d_boys,   c->d_sph,   c->d_D,     c->d_Ds,    c->d_Fh, c->d_io,
                   c->d_dmax,  c->d_cnt,    c->d_qoff,   c->d_wmap_i, c->d_wmap_c, c->d_wmeta, c->d_wdims, c->d_gw,
                   c->d_shinfo, c->d_blk_gab, c->d_blk_info, c->d_blk_dmax, c->d_ks_i, c->d_ks_q, c->d_ks_pp,
-                  c->d_store};
+                  c->d_store, c->d_fine,   c->d_row_bra, c->d_row_tasks, c->d_row_work,
+                  c->d_one,   c->d_pg};
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  for (double *p : c->d_frag)
+    if (p) cudaFree(p);
+  for (dgf_graph &gr : c->graphs)
+    if (gr.exec) cudaGraphExecDestroy(gr.exec);
+  for (int k = 1; k < kForkStreams; ++k) {
+    if (c->fork[k]) cudaStreamDestroy(c->fork[k]);
+    if (c->ev_join[k]) cudaEventDestroy(c->ev_join[k]);
+  }
+  if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->stream) cudaStreamDestroy(c->stream);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
@@ -150,6 +201,40 @@ static void free_ctx(dgf_ctx *c) {
 
 
 static int cls_l1(int X) { return (X == 0) ? 0 : (X <= 2) ? 1 : (X <= 5) ? 2 : 3; }
+static int pair_l(int X) { return cls_l1(X) + (X - cls_l1(X) * (cls_l1(X) + 1) / 2); }  // la + lb
+
+// The kernel of plan entry cp in an FP64 launch that is not a half of a mixed
+// split: the row kernel (one density slot), the pack kernel, or the others.
+// Sharded builds ignore what the tuner chose here, so that every rank cuts
+// the entry the same way.
+//
+// The row kernel takes spherical functions (classes of s and p have no
+// others), kets from the ket table and 32-bit matrix offsets.
+static bool row_ok(const dgf_ctx *c, const ClassPlan &cp) {
+  const bool sph = c->spherical || (cls_l1(cp.X) < 2 && cls_l1(cp.Y) < 2);
+  return cp.row_ntask > 0 && sph && c->d_ks_i && c->nwf <= 46340 && jk_row_entry(cp.X, cp.Y).launch;
+}
+
+// The pack kernel: spherical functions, pair fragments made.
+static bool pack_ok(const dgf_ctx *c, const ClassPlan &cp) {
+  return cp.row_ntask > 0 && c->spherical && g_pack_table[cp.X][cp.Y].launch && c->d_frag[cp.X] && c->d_frag[cp.Y];
+}
+
+enum { kRouteOther = 0, kRouteRow = 1, kRoutePack = 2 };
+static int class_route(const dgf_ctx *c, const ClassPlan &cp, int nslot, bool sharded) {
+  const int v = sharded ? kDefaultVariant : c->choice[cp.X][cp.Y][0];
+  const bool row = nslot == 1 && row_ok(c, cp), pack = pack_ok(c, cp);
+  if (v == kPackVariant && pack) return kRoutePack;
+  if (v == kRowVariant && row) return kRouteRow;
+  if (v != kDefaultVariant && v != kPackVariant && v != kRowVariant) return kRouteOther;
+  if (pack && g_pack_table[cp.X][cp.Y].preferred) return kRoutePack;
+  return row ? kRouteRow : kRouteOther;
+}
+
+// Whether the mixed form splits an untuned class although a pack kernel has it.
+static bool keeps_split(const dgf_ctx *c, const ClassPlan &cp, int route) {
+  return route == kRoutePack && c->split_ok[cp.X][cp.Y] == 1 && pair_l(cp.X) + pair_l(cp.Y) >= 7;
+}
 
 // Kernel for class pair (X, Y): precision 0 = FP64 (the context's choice),
 // 1 = FP32 thread kernel, 2 = FP64 team kernel (Schwarz pre-pass).
@@ -164,7 +249,7 @@ static const ClassKernel &select_kernel(const dgf_ctx *c, int X, int Y, int prec
 }
 
 static int launch_kernel(dgf_ctx *c, const ClassKernel &k, int X, int Y, JKArgs &args, cudaStream_t st,
-                         int precision);
+                         int precision, const PackArgs *pk = nullptr);
 
 static int launch_class(dgf_ctx *c, int X, int Y, JKArgs &args, cudaStream_t st, int precision,
                         bool ket1 = false) {
@@ -172,14 +257,28 @@ static int launch_class(dgf_ctx *c, int X, int Y, JKArgs &args, cudaStream_t st,
 }
 
 static int launch_kernel(dgf_ctx *c, const ClassKernel &k, int X, int Y, JKArgs &args, cudaStream_t st,
-                         int precision) {
-  if (!k.launch) DGF_FAIL(DGF_ERR_UNSUPPORTED, "no kernel for this class and precision");
+                         int precision, const PackArgs *pk) {
+  const bool tasks = k.kind == kKindRow || k.kind == kKindPack;
+  if (!k.launch && !pk) DGF_FAIL(DGF_ERR_UNSUPPORTED, "no kernel for this class and precision");
   const bool thread_kernel = (k.kind == kKindThread);
+  if (tasks) {
+    if (args.row_task1 <= args.row_task0) return DGF_OK;
+    if (c->row_slot >= kRowSlots) {
+      DGF_CUDA_CHECK(cudaMemsetAsync(c->d_row_work, 0, (size_t)kRowSlots * kRowChunksMax * sizeof(unsigned), st));
+      c->row_slot = 0;
+    }
+    args.row_work = c->d_row_work + (size_t)kRowChunksMax * c->row_slot++;
+  }
   const int64_t per_block = k.qpb;  // thread kernels: a quartet per thread; team kernels: per block or per warp
   const int64_t nq = args.nquartet - args.q_begin;
   if (nq <= 0 && !args.diag_out) return DGF_OK;
   int64_t grid64 = std::min<int64_t>((nq + per_block - 1) / per_block, (int64_t)c->nsm * (thread_kernel ? 8 : 16));
   int grid = (int)std::max<int64_t>(grid64, 1);
+  if (tasks) {  // resident blocks, over the A chunks, no more than there are tasks for
+    const int64_t warps = k.block / 32;
+    grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)args.row_task1 - args.row_task0 + warps - 1) / warps,
+                                                       ((int64_t)c->nsm * k.qpb + k.chunks - 1) / k.chunks));
+  }
   const bool prof = c->profiling && !args.diag_out;
   if (prof) {
     cudaEvent_t e0, e1;
@@ -189,7 +288,10 @@ static int launch_kernel(dgf_ctx *c, const ClassKernel &k, int X, int Y, JKArgs 
     c->prof_ev.push_back(e1);
     DGF_CUDA_CHECK(cudaEventRecord(e0, st));
   }
-  k.launch(args, grid, k.block, k.smem, st);
+  if (pk)
+    g_pack_table[X][Y].launch(args, *pk, grid, st);
+  else
+    k.launch(args, grid, k.block, k.smem, st);
   DGF_CUDA_CHECK(cudaGetLastError());
   if (prof) {
     DGF_CUDA_CHECK(cudaEventRecord(c->prof_ev.back(), st));
@@ -203,6 +305,8 @@ static int launch_kernel(dgf_ctx *c, const ClassKernel &k, int X, int Y, JKArgs 
                : k.kind == kKindWarpTeam   ? 2
                : k.kind == kKindWarp       ? 4
                : k.kind == kKindWarpMma    ? 6
+               : k.kind == kKindRow        ? 8
+               : k.kind == kKindPack       ? 10
                                            : 1;
     (void)k;
     r.quartets = args.nquartet - args.q_begin;
@@ -445,7 +549,7 @@ static int build_working_basis(dgf_ctx *c, const dgf_basis *b) {
     const int at = (int)b->block_atom[ib], nf = nfun(l, c->spherical);
     const double *cf = b->coef + b->block_coef_offset[ib];  // column-major (np, nc)
     const double *ex = b->prim_exp + b->block_prim_offset[ib];
-    bool general = false;
+    bool general = c->resolve_all && np > 1;
     for (int i = 0; i < np && !general; ++i) {
       int used = 0;
       for (int k = 0; k < nc; ++k) used += (cf[(size_t)k * np + i] != 0.0);
@@ -557,7 +661,10 @@ static int upload_working_maps(dgf_ctx *c) {
   if (!shinfo.empty())
     DGF_CUDA_CHECK(cudaMemcpy(c->d_shinfo, shinfo.data(), shinfo.size() * sizeof(int), cudaMemcpyHostToDevice));
   for (int X = 0; X < kNumPairClass; ++X)
-    for (int Y = 0; Y < kNumPairClass; ++Y) c->split_ok[X][Y] = 1;
+    for (int Y = 0; Y < kNumPairClass; ++Y) {
+      c->split_ok[X][Y] = 1;
+      c->choice[X][Y][0] = c->choice[X][Y][1] = kDefaultVariant;
+    }
   return DGF_OK;
 }
 
@@ -574,7 +681,65 @@ extern "C" void dgf_default_options(dgf_options *opt) {
   opt->hfxatt = 0.0;
 }
 
-extern "C" int dgf_create(const dgf_basis *b, int device, dgf_ctx **out) {
+// Working functions a resolved context may have: the largest size every entry
+// point takes (dgf_fock_device_noalloc's fixed scratch).
+constexpr int kPrimMaxW = 1536;
+
+// Keeps a copy of the basis where contracted shells could be resolved.
+static void keep_basis(dgf_ctx *c, const dgf_basis *b) {
+  if (c->resolve_all) return;
+  bool contracted = false;
+  for (int n : c->ws_nprim) contracted = contracted || n > 1;
+  if (!contracted) return;
+  int64_t nw = 0, nprim = 0, ncoef = 0;
+  for (dgf_int i = 0; i < b->nblock; ++i) {
+    const dgf_int np = b->block_nprim[i], nc = b->block_ncontr[i];
+    nw += (np > 1 ? np : nc) * nfun((int)b->block_l[i], c->spherical);
+    nprim = std::max<int64_t>(nprim, b->block_prim_offset[i] + np);
+    ncoef = std::max<int64_t>(ncoef, b->block_coef_offset[i] + np * nc);
+  }
+  if (nw > kPrimMaxW) return;
+  c->prim_fits = true;
+  const size_t nb = (size_t)b->nblock;
+  const dgf_int *src[7] = {b->block_l, b->block_atom, b->block_nprim, b->block_ncontr,
+                           b->block_ao_offset, b->block_prim_offset, b->block_coef_offset};
+  for (const dgf_int *p : src) c->basis_i.insert(c->basis_i.end(), p, p + nb);
+  c->basis_d.insert(c->basis_d.end(), b->prim_exp, b->prim_exp + nprim);
+  c->basis_d.insert(c->basis_d.end(), b->coef, b->coef + ncoef);
+  c->basis_d.insert(c->basis_d.end(), b->atom_xyz, b->atom_xyz + 3 * b->natom);
+  c->basis_d.insert(c->basis_d.end(), b->atom_charge, b->atom_charge + b->natom);
+  dgf_basis &k = c->basis_copy;
+  k = *b;
+  const dgf_int *i = c->basis_i.data();
+  k.block_l = i;
+  k.block_atom = i + nb;
+  k.block_nprim = i + 2 * nb;
+  k.block_ncontr = i + 3 * nb;
+  k.block_ao_offset = i + 4 * nb;
+  k.block_prim_offset = i + 5 * nb;
+  k.block_coef_offset = i + 6 * nb;
+  const double *d = c->basis_d.data();
+  k.prim_exp = d;
+  k.coef = d + nprim;
+  k.atom_xyz = d + nprim + ncoef;
+  k.atom_charge = d + nprim + ncoef + 3 * b->natom;
+}
+
+static int create_ctx(const dgf_basis *b, int device, bool resolve_all, dgf_ctx **out);
+
+dgf_ctx *direct_ctx(dgf_ctx *c) {
+  if (!c->prim_fits || c->user_tuned) return c;
+  if (!c->prim && create_ctx(&c->basis_copy, c->device, true, &c->prim) != DGF_OK) {
+    c->prim = nullptr;  // no memory for it: the contracted form serves
+    c->prim_fits = false;
+    return c;
+  }
+  return c->prim;
+}
+
+extern "C" int dgf_create(const dgf_basis *b, int device, dgf_ctx **out) { return create_ctx(b, device, false, out); }
+
+static int create_ctx(const dgf_basis *b, int device, bool resolve_all, dgf_ctx **out) {
   if (!out) DGF_FAIL(DGF_ERR_ARG, "out is NULL");
   *out = nullptr;
   if (!b || b->nblock <= 0 || b->natom <= 0 || b->nbf <= 0) DGF_FAIL(DGF_ERR_ARG, "empty or invalid basis");
@@ -590,10 +755,9 @@ extern "C" int dgf_create(const dgf_basis *b, int device, dgf_ctx **out) {
   if (device < 0 || device >= ndev) DGF_FAIL(DGF_ERR_ARG, "device index out of range");
   std::unique_ptr<dgf_ctx, void (*)(dgf_ctx *)> c(new dgf_ctx, free_ctx);
   c->device = device;
+  c->resolve_all = resolve_all;
   DeviceGuard g(device);
-  cudaDeviceProp prop;
-  DGF_CUDA_CHECK(cudaGetDeviceProperties(&prop, device));
-  c->nsm = prop.multiProcessorCount;
+  DGF_CUDA_CHECK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device));
   c->nbf = (int)b->nbf;
   c->natom = (int)b->natom;
   c->spherical = b->spherical ? 1 : 0;
@@ -636,6 +800,7 @@ extern "C" int dgf_create(const dgf_basis *b, int device, dgf_ctx **out) {
   // Two-electron working basis and its map to the AO basis.
   int st_wb = build_working_basis(c.get(), b);
   if (st_wb) return st_wb;
+  keep_basis(c.get(), b);
 
   // Dalton blocks: working shells per block (a block that is one working
   // shell is "whole"), and each block's AO functions.
@@ -661,18 +826,28 @@ extern "C" int dgf_create(const dgf_basis *b, int device, dgf_ctx **out) {
   DGF_CUDA_CHECK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   DGF_CUDA_CHECK(cudaEventCreate(&c->ev0));
   DGF_CUDA_CHECK(cudaEventCreate(&c->ev1));
+  DGF_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+  for (int k = 1; k < kForkStreams; ++k) {
+    DGF_CUDA_CHECK(cudaStreamCreateWithFlags(&c->fork[k], cudaStreamNonBlocking));
+    DGF_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_join[k], cudaEventDisableTiming));
+  }
   DGF_CUDA_CHECK(jk_prepare_all());
-  std::vector<double> boys, sph;
-  boys_table_host(boys);
+  // the Boys tables hold constants only: made once per process
+  static const std::vector<double> boys = [] { std::vector<double> v; boys_table_host(v); return v; }();
+  static const std::vector<double> fine = [] { std::vector<double> v; boys_fine_host(v); return v; }();
+  std::vector<double> sph;
   sph_table_host(sph);
   if (dev_alloc(&c->d_boys, boys.size()) != cudaSuccess || dev_alloc(&c->d_sph, sph.size()) != cudaSuccess ||
       dev_alloc(&c->d_pp, c->pp.size()) != cudaSuccess || dev_alloc(&c->d_pairs, c->pairs.size()) != cudaSuccess ||
-      dev_alloc(&c->d_cnt, 4 * kCounterSlots) != cudaSuccess) {
+      dev_alloc(&c->d_cnt, 4 * kCounterSlots) != cudaSuccess || dev_alloc(&c->d_fine, fine.size()) != cudaSuccess ||
+      dev_alloc(&c->d_row_bra, c->pairs.size()) != cudaSuccess ||
+      dev_alloc(&c->d_row_work, (size_t)kRowSlots * kRowChunksMax) != cudaSuccess) {
     cudaGetLastError();
     DGF_FAIL(DGF_ERR_NOMEM, "device allocation failed while creating the context");
   }
   DGF_CUDA_CHECK(cudaMemcpy(c->d_boys, boys.data(), boys.size() * 8, cudaMemcpyHostToDevice));
   DGF_CUDA_CHECK(cudaMemcpy(c->d_sph, sph.data(), sph.size() * 8, cudaMemcpyHostToDevice));
+  DGF_CUDA_CHECK(cudaMemcpy(c->d_fine, fine.data(), fine.size() * 8, cudaMemcpyHostToDevice));
   DGF_CUDA_CHECK(cudaMemcpy(c->d_pp, c->pp.data(), c->pp.size() * sizeof(PrimPair), cudaMemcpyHostToDevice));
   DGF_CUDA_CHECK(
       cudaMemcpy(c->d_pairs, c->pairs.data(), c->pairs.size() * sizeof(PairRec), cudaMemcpyHostToDevice));
@@ -719,6 +894,22 @@ extern "C" int dgf_create(const dgf_basis *b, int device, dgf_ctx **out) {
   DGF_CUDA_CHECK(cudaMemcpy(c->d_pp, c->pp.data(), c->pp.size() * sizeof(PrimPair), cudaMemcpyHostToDevice));
   DGF_CUDA_CHECK(
       cudaMemcpy(c->d_pairs, c->pairs.data(), c->pairs.size() * sizeof(PairRec), cudaMemcpyHostToDevice));
+  // Bra pairs of every class in row order.
+  c->row_bra.resize(c->pairs.size());
+  for (int X = 0; X < kNumPairClass; ++X) {
+    const int o = c->cls_off[X], n = c->cls_off[X + 1] - o;
+    int *rb = c->row_bra.data() + o;
+    for (int i = 0; i < n; ++i) rb[i] = i;
+    const PairRec *pr = c->pairs.data() + o;
+    std::sort(rb, rb + n, [pr](int u, int v) {
+      if (pr[u].shA != pr[v].shA) return pr[u].shA < pr[v].shA;
+      const int bu = npp_bucket(pr[u].npp), bv = npp_bucket(pr[v].npp);
+      if (bu != bv) return bu < bv;
+      return pr[u].Q != pr[v].Q ? pr[u].Q > pr[v].Q : u < v;
+    });
+  }
+  if (!c->row_bra.empty())
+    DGF_CUDA_CHECK(cudaMemcpy(c->d_row_bra, c->row_bra.data(), c->row_bra.size() * sizeof(int), cudaMemcpyHostToDevice));
   // Ket table of single-primitive kets (first primitive pair of every pair).
   if (c->nwshell < 65536 && !c->pairs.empty()) {
     const size_t np = c->pairs.size();
@@ -832,10 +1023,103 @@ static void set_ket_table(const dgf_ctx *c, const ClassPlan &cp, JKArgs &a) {
   a.ks_base = c->cls_off[cp.Y] + cp.kb0;
 }
 
+// Row-kernel arguments of a plan entry, tasks [t0, t1).
+static void set_row_args(const dgf_ctx *c, const ClassPlan &cp, JKArgs &a, int t0, int t1) {
+  const int L = pair_l(cp.X) + pair_l(cp.Y);  // the row kernels' orders only
+  a.boys_fine = L <= kFineMaxM ? c->d_fine + (size_t)L * kFineDoubles : nullptr;
+  a.row_bra = c->d_row_bra + c->cls_off[cp.X];
+  a.row_tasks = c->d_row_tasks + cp.row_off;
+  a.row_task0 = t0;
+  a.row_task1 = t1;
+}
+
+// Tasks of the row kernels: a source's bras in row order, cut into segments
+// of at most R bras of one A shell, each with the 32-ket chunks its longest
+// prefix reaches, at most G chunks a task: {first bra, bras | chunks << 16,
+// first ket, end of the kets}.  R starts at max_bras and is halved while that
+// leaves fewer segment-chunks than about one per resident warp of the GPU (a
+// segment's tile then has fewer bras to spread its own atomics over, but a
+// small molecule would leave most warps without work); G, at most 16, leaves
+// every warp several tasks.  min_width < 32 (pack kernels, whose warps work
+// through a chunk's kets one after the other): chunks too are halved, down to
+// that, while there are too few.  Depends on the molecules and the threshold only,
+// so that every rank of a sharded build makes the same list.
+void row_tasks(const std::vector<RowSource> &src, int max_bras, int min_width, std::vector<int4> &tasks) {
+  const int64_t units_want = 148 * 10, tasks_want = 148 * 12 * 4;
+  int width = 32;
+  auto segments = [&](int R, auto f) {
+    for (const RowSource &s : src)
+      for (int i = 0; i < s.n;) {
+        int j = i, most = 0;
+        while (j < s.n && j - i < R && s.pairs[s.order[j]].shA == s.pairs[s.order[i]].shA) {
+          most = std::max(most, (int)(s.qoff[s.order[j] + 1] - s.qoff[s.order[j]]));
+          ++j;
+        }
+        if (most > 0) f(s, i, j - i, (most + width - 1) / width);
+        i = j;
+      }
+  };
+  auto units = [&](int R) {
+    int64_t u = 0;
+    segments(R, [&](const RowSource &, int, int, int nch) { u += nch; });
+    return u;
+  };
+  int R = max_bras;
+  int64_t u = units(R);
+  while (R > 1 && u < units_want) u = units(R /= 2);
+  while (width > min_width && u < units_want) {
+    width /= 2;
+    u = units(R);
+  }
+  const int G = (int)std::min<int64_t>(16, std::max<int64_t>(1, u / tasks_want));
+  segments(R, [&](const RowSource &s, int b0, int nb, int nch) {
+    for (int ch = 0; ch < nch; ch += G) {
+      const int k0 = s.ket0 + width * ch, end = width < 32 ? std::min(k0 + width, s.ket_end) : s.ket_end;
+      tasks.push_back(make_int4(s.bra0 + b0, nb | (std::min(G, nch - ch) << 16), k0, end));
+    }
+  });
+}
+
+static int launch_pack(dgf_ctx *c, const ClassPlan &cp, JKArgs &a, cudaStream_t st) {
+  const PackEntry &e = g_pack_table[cp.X][cp.Y];
+  const PackArgs pk{c->d_frag[cp.X], c->d_frag[cp.Y] + (size_t)cp.kb0 * g_frag_table[cp.Y].doubles};
+  const ClassKernel k{nullptr, 32 * e.wpb, 0, 1, e.blocks, kKindPack};
+  return launch_kernel(c, k, cp.X, cp.Y, a, st, 0, &pk);
+}
+
+// Pair fragments of the classes the plan's pack kernels read, once per
+// context.  Without the memory for them the classes keep their other kernels.
+static int ensure_frags(dgf_ctx *c, const std::vector<ClassPlan> &plan) {
+  if (!c->spherical) return DGF_OK;
+  bool need[kNumPairClass] = {}, made = false;
+  for (const ClassPlan &cp : plan)
+    if (cp.row_ntask > 0 && g_pack_table[cp.X][cp.Y].launch) need[cp.X] = need[cp.Y] = true;
+  size_t total = 0;
+  for (int X = 0; X < kNumPairClass; ++X)
+    if (need[X] || c->d_frag[X]) total += (size_t)(c->cls_off[X + 1] - c->cls_off[X]) * g_frag_table[X].doubles * 8;
+  if (total > kFragMaxBytes) return DGF_OK;
+  for (int X = 0; X < kNumPairClass; ++X) {
+    const int n = c->cls_off[X + 1] - c->cls_off[X];
+    if (!need[X] || c->d_frag[X] || !n) continue;
+    if (dev_alloc(&c->d_frag[X], (size_t)n * g_frag_table[X].doubles) != cudaSuccess) {
+      cudaGetLastError();
+      c->d_frag[X] = nullptr;
+      continue;
+    }
+    g_frag_table[X].launch(c->d_pairs + c->cls_off[X], c->d_pp, n, c->d_sph, c->d_frag[X],
+                           std::min((n + 3) / 4, c->nsm * 16), c->stream);
+    made = true;
+  }
+  DGF_CUDA_CHECK(cudaGetLastError());
+  if (made) DGF_CUDA_CHECK(cudaStreamSynchronize(c->stream));
+  return DGF_OK;
+}
+
 static int build_plan(dgf_ctx *c, double thrs) {
   if (c->plan_thrs == thrs && !c->plan.empty()) return DGF_OK;
   std::vector<int64_t> all;
   std::vector<ClassPlan> plan;
+  std::vector<int4> tasks;
   for (int X = 0; X < kNumPairClass; ++X)
     for (int Y = 0; Y <= X; ++Y) {
       const int nb = c->cls_off[X + 1] - c->cls_off[X], nk = c->cls_off[Y + 1] - c->cls_off[Y];
@@ -870,9 +1154,33 @@ static int build_plan(dgf_ctx *c, double thrs) {
           all.push_back(acc);
         }
         cp.nquartet = acc;
-        if (acc > 0) plan.push_back(cp);
+        if (acc > 0) {
+          // the row and pack kernels take single-primitive pairs on both
+          // sides; the gradient's cover s, p and d bras
+          if (kb == 0 && c->cls_max_npp[X] == 1 &&
+              (cls_l1(X) <= 2 || jk_row_entry(X, Y).launch || g_pack_table[X][Y].launch)) {
+            cp.row_off = (int64_t)tasks.size();
+            row_tasks({RowSource{c->row_bra.data() + c->cls_off[X], nb, bra, &all[cp.off], 0, 0, k1 - k0}},
+                      row_max_bras(X), g_pack_table[X][Y].launch && g_pack_table[X][Y].preferred ? 4 : 32, tasks);
+            cp.row_ntask = (int)(tasks.size() - cp.row_off);
+          }
+          plan.push_back(cp);
+        }
       }
     }
+  if (tasks.size() > c->row_tasks_cap) {
+    if (c->d_row_tasks) cudaFree(c->d_row_tasks);
+    c->d_row_tasks = nullptr;
+    c->row_tasks_cap = 0;
+    c->plan.clear();
+    if (dev_alloc(&c->d_row_tasks, tasks.size()) != cudaSuccess) {
+      cudaGetLastError();
+      DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the row tasks failed");
+    }
+    c->row_tasks_cap = tasks.size();
+  }
+  if (!tasks.empty())
+    DGF_CUDA_CHECK(cudaMemcpy(c->d_row_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice));
   if (all.size() > c->qoff_cap) {
     if (c->d_qoff) cudaFree(c->d_qoff);
     c->d_qoff = nullptr;
@@ -884,8 +1192,10 @@ static int build_plan(dgf_ctx *c, double thrs) {
     c->qoff_cap = all.size();
   }
   DGF_CUDA_CHECK(cudaMemcpy(c->d_qoff, all.data(), all.size() * 8, cudaMemcpyHostToDevice));
+  if (const int r = ensure_frags(c, plan)) return r;
   c->plan.swap(plan);
   c->plan_thrs = thrs;
+  ++c->gen;
   return DGF_OK;
 }
 
@@ -893,6 +1203,7 @@ int dgf_plan_for(dgf_ctx *c, double thrs) { return build_plan(c, thrs); }
 
 static int ensure_slots(dgf_ctx *c, int nslot) {
   if (nslot <= c->cap_slots) return DGF_OK;
+  ++c->gen;
   const size_t n2 = (size_t)c->nwf * c->nwf;
   for (double **p : {&c->d_D, &c->d_Ds, &c->d_Fh}) {
     if (*p) cudaFree(*p);
@@ -1014,6 +1325,7 @@ static int ensure_block_screen(dgf_ctx *c, int nslot) {
     DGF_CUDA_CHECK(cudaMemcpy(c->d_blk_info, info.data(), info.size() * sizeof(int), cudaMemcpyHostToDevice));
   }
   if (nslot > c->cap_blk_slots) {
+    ++c->gen;
     if (c->d_blk_dmax) cudaFree(c->d_blk_dmax);
     c->d_blk_dmax = nullptr;
     c->cap_blk_slots = 0;
@@ -1087,6 +1399,38 @@ static void shard_range(const dgf_ctx *c, size_t e, int64_t r, int64_t n, int64_
 static int64_t store_nint(const dgf_ctx *c, int X, int Y) {
   const int la = cls_l1(X), lb = X - la * (la + 1) / 2, lc = cls_l1(Y), ld = Y - lc * (lc + 1) / 2;
   return (int64_t)nfun(la, c->spherical) * nfun(lb, c->spherical) * nfun(lc, c->spherical) * nfun(ld, c->spherical);
+}
+
+// Builds estimated to take less than this are replayed as graphs: below it
+// the host's launches (about 3 us each, two dozen or more) are a visible part
+// of the call; above it an instantiated graph would only hold memory.
+constexpr double kGraphSeconds = 5e-3;
+constexpr size_t kGraphCache = 4;  // option sets a context keeps a graph for
+
+static void drop_graphs(dgf_ctx *c) {
+  for (dgf_graph &g : c->graphs)
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+  c->graphs.clear();
+}
+
+// The context's record of a build with these options, most recent first;
+// `seen` counts its calls.
+static dgf_graph *graph_entry(dgf_ctx *c, const std::string &key) {
+  if (c->graph_gen != c->gen) drop_graphs(c);  // plan, buffers or kernel choices changed
+  c->graph_gen = c->gen;
+  size_t i = 0;
+  while (i < c->graphs.size() && c->graphs[i].key != key) ++i;
+  if (i == c->graphs.size()) {
+    if (c->graphs.size() == kGraphCache) {
+      if (c->graphs.back().exec) cudaGraphExecDestroy(c->graphs.back().exec);
+      c->graphs.pop_back();
+    }
+    c->graphs.insert(c->graphs.begin(), dgf_graph{key, nullptr, 0, 0});
+  } else if (i > 0) {
+    std::rotate(c->graphs.begin(), c->graphs.begin() + i, c->graphs.begin() + i + 1);
+  }
+  ++c->graphs[0].seen;
+  return &c->graphs[0];
 }
 
 // stored = true: the conventional form, digesting the blocks of the integral
@@ -1169,14 +1513,14 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
     c->prof_ev.clear();
     c->prof.clear();
   }
-  DGF_CUDA_CHECK(cudaMemsetAsync(c->d_cnt, 0, 4 * kCounterSlots * sizeof(unsigned long long), st));
-  DGF_CUDA_CHECK(cudaEventRecord(c->ev0, st));
-  int64_t launches = 0, total_q = 0, nlaunch_class = 0;
-  std::vector<int64_t> sq0(c->plan.size()), sq1(c->plan.size());
-  for (size_t e = 0; e < c->plan.size(); ++e) {
-    shard_range(c, e, o.shard_index, o.shard_count, &sq0[e], &sq1[e]);
-    total_q += sq1[e] - sq0[e];
+  const bool count = stats || c->profiling;  // the kernels count quartets only for a caller that reads the counts
+  if (count) {
+    DGF_CUDA_CHECK(cudaMemsetAsync(c->d_cnt, 0, 4 * kCounterSlots * sizeof(unsigned long long), st));
+    DGF_CUDA_CHECK(cudaEventRecord(c->ev0, st));
   }
+  int64_t launches = 0, nlaunch_class = 0;
+  std::vector<int64_t> sq0(c->plan.size()), sq1(c->plan.size());
+  for (size_t e = 0; e < c->plan.size(); ++e) shard_range(c, e, o.shard_index, o.shard_count, &sq0[e], &sq1[e]);
   // Zero outputs that have no contributions.
   for (int k = 0; k < ndmat; ++k)
     if (outs[k].zero) DGF_CUDA_CHECK(cudaMemsetAsync(fmat_dev + (size_t)k * n2ao, 0, n2ao * 8, st));
@@ -1190,7 +1534,6 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
                        (int64_t)n2, c->nsm, st);
       ++launches;
     }
-    DGF_CUDA_CHECK(cudaMemsetAsync(c->d_Fh, 0, ns * n2 * 8, st));
     if (need_dmax) {
       dmax_kernel<<<std::max(1, std::min(nws * nws / 128 + 1, c->nsm * 8)), 128, 0, st>>>(
           c->d_D, ns, N, d_shinfo, d_shinfo + nws, nws, c->d_dmax);
@@ -1222,62 +1565,179 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
     a.split = o.mixed_cutoff;
     a.schwarz_thr = o.thrs;
     a.mode = 0;
-    // Pass 0: 1/r12 with the slots' Coulomb and exchange scales; pass 1
-    // (range-separated exchange): erf(mu r12)/r12, exchange only.
+    // The launches of this chunk.  Pass 0: 1/r12 with the slots' Coulomb and
+    // exchange scales; pass 1 (range-separated exchange): erf(mu r12)/r12,
+    // exchange only.
+    struct Item {
+      size_t e;
+      int pass;
+      double s;  // estimated time
+    };
+    std::vector<Item> items;
+    double seconds = 0.0;
     for (int pass = 0; pass < (attenuated ? 2 : 1); ++pass) {
       bool any = false;
-      for (int s = 0; s < ns; ++s) {
-        a.jscale[s] = pass == 0 ? slots[s0 + s].js : 0.0;
-        a.kscale[s] = pass == 0 ? slots[s0 + s].ks : slots[s0 + s].ka;
-        any = any || a.jscale[s] != 0.0 || a.kscale[s] != 0.0;
-      }
-      a.erf_mu2 = pass == 0 ? 0.0 : o.hfxmu * o.hfxmu;
+      for (int s = 0; s < ns; ++s)
+        any = any || (pass == 0 ? slots[s0 + s].js != 0.0 || slots[s0 + s].ks != 0.0 : slots[s0 + s].ka != 0.0);
       if (!any) continue;
       for (size_t e = 0; e < c->plan.size(); ++e) {
-        const ClassPlan &cp = c->plan[e];
         if (sq1[e] <= sq0[e]) continue;  // not in this shard
-        a.bra = c->d_pairs + c->cls_off[cp.X];
-        a.ket = c->d_pairs + c->cls_off[cp.Y] + cp.kb0;
-        a.ket_off = cp.kb0;
-        a.ket_pp0 = ket_pp0_of(c, cp);
-        set_ket_table(c, cp, a);
-        a.nbra = c->cls_off[cp.X + 1] - c->cls_off[cp.X];
-        a.same_class = (cp.X == cp.Y);
-        a.qoff = c->d_qoff + cp.off;
-        a.q_begin = sq0[e];
-        a.nquartet = sq1[e];
-        // Boys table of order L = la+lb+lc+ld.
-        const int la = (cp.X == 0) ? 0 : (cp.X <= 2) ? 1 : (cp.X <= 5) ? 2 : 3;
-        const int lb = cp.X - la * (la + 1) / 2;
-        const int lc = (cp.Y == 0) ? 0 : (cp.Y <= 2) ? 1 : (cp.Y <= 5) ? 2 : 3;
-        const int ld = cp.Y - lc * (lc + 1) / 2;
-        a.boys = c->d_boys + (size_t)(la + lb + lc + ld) * kBoysTableDoubles;
-        const bool split = o.mixed_cutoff > 0.0 && c->split_ok[cp.X][cp.Y] &&
-                           select_kernel(c, cp.X, cp.Y, 1, cp.bucket == 0).launch != nullptr;
-        const int Lq = la + lb + lc + ld;
-        if (stored) {  // conventional form: digest the stored blocks
-          a.store_in = c->d_store;
-          a.store_base = c->store_off[e];
-          a.store_nint = (int)store_nint(c, cp.X, cp.Y);
-          a.mode = 0;
-          a.counters = c->d_cnt + 4 * (nlaunch_class % kCounterSlots);
-          ++nlaunch_class;
-          int r = launch_kernel(c, jk_stored_kernel(cp.X, cp.Y), cp.X, cp.Y, a, st, 0);
-          if (r) return r;
-          ++launches;
-          continue;
-        }
-        for (int part = 0; part < (split ? 2 : 1); ++part) {
-          a.mode = split ? 1 + part : 0;
-          // the FP32 half reads the low-degree Boys table
-          a.boys = c->d_boys + ((split && part == 1) ? boys_low_offset(Lq) : (size_t)Lq * kBoysTableDoubles);
-          a.counters = c->d_cnt + 4 * (nlaunch_class % kCounterSlots);
-          ++nlaunch_class;
-          int r = launch_class(c, cp.X, cp.Y, a, st, split && part == 1 ? 1 : 0, cp.bucket == 0);
-          if (r) return r;
-          ++launches;
-        }
+        // model operations at 5 TFLOP/s, plus the time one quartet takes alone
+        const double t = (double)(sq1[e] - sq0[e]) * entry_cost_per_quartet(c, c->plan[e]) / 5e12 + 6e-6 +
+                         2e-7 * n3(pair_l(c->plan[e].X) + pair_l(c->plan[e].Y));
+        items.push_back({e, pass, t});
+        seconds += t;
       }
+    }
+    auto enqueue = [&](const Item &it, cudaStream_t ls) -> int {
+      const size_t e = it.e;
+      const ClassPlan &cp = c->plan[e];
+      for (int s = 0; s < ns; ++s) {
+        a.jscale[s] = it.pass == 0 ? slots[s0 + s].js : 0.0;
+        a.kscale[s] = it.pass == 0 ? slots[s0 + s].ks : slots[s0 + s].ka;
+      }
+      a.erf_mu2 = it.pass == 0 ? 0.0 : o.hfxmu * o.hfxmu;
+      a.bra = c->d_pairs + c->cls_off[cp.X];
+      a.ket = c->d_pairs + c->cls_off[cp.Y] + cp.kb0;
+      a.ket_off = cp.kb0;
+      a.ket_pp0 = ket_pp0_of(c, cp);
+      set_ket_table(c, cp, a);
+      a.nbra = c->cls_off[cp.X + 1] - c->cls_off[cp.X];
+      a.same_class = (cp.X == cp.Y);
+      a.qoff = c->d_qoff + cp.off;
+      a.q_begin = sq0[e];
+      a.nquartet = sq1[e];
+      a.mode = 0;
+      const int Lq = pair_l(cp.X) + pair_l(cp.Y);  // the Boys tables are by order
+      a.boys = c->d_boys + (size_t)Lq * kBoysTableDoubles;
+      auto set_task_range = [&](JKArgs &ra) {
+        // a shard's tasks: the same fractions of the entry's list as of its quartets
+        const double f = (double)cp.row_ntask / (double)cp.nquartet;
+        const int t0 = (int)((double)sq0[e] * f);
+        const int t1 = sq1[e] == cp.nquartet ? cp.row_ntask : (int)((double)sq1[e] * f);
+        set_row_args(c, cp, ra, t0, t1);
+      };
+      auto counters = [&]() { return count ? c->d_cnt + 4 * (nlaunch_class % kCounterSlots) : nullptr; };
+      if (stored) {  // conventional form: digest the stored blocks
+        a.store_in = c->d_store;
+        a.store_base = c->store_off[e];
+        a.store_nint = (int)store_nint(c, cp.X, cp.Y);
+        a.counters = counters();
+        ++nlaunch_class;
+        ++launches;
+        if (ns == 1 && row_ok(c, cp)) {
+          set_task_range(a);
+          return launch_kernel(c, g_row_stored[cp.X][cp.Y], cp.X, cp.Y, a, ls, 0);
+        }
+        return launch_kernel(c, jk_stored_kernel(cp.X, cp.Y), cp.X, cp.Y, a, ls, 0);
+      }
+      const int route = class_route(c, cp, ns, o.shard_count > 1);
+      const bool row = route != kRouteOther;
+      // a class with a row kernel splits only where the tuner saw it win
+      const bool split = o.mixed_cutoff > 0.0 &&
+                         (row ? o.shard_count == 1 && (c->split_ok[cp.X][cp.Y] == 2 || keeps_split(c, cp, route))
+                              : c->split_ok[cp.X][cp.Y] != 0) &&
+                         select_kernel(c, cp.X, cp.Y, 1, cp.bucket == 0).launch != nullptr;
+      if (row && !split) {
+        set_task_range(a);
+        a.counters = counters();
+        ++nlaunch_class;
+        ++launches;
+        if (route == kRoutePack) return launch_pack(c, cp, a, ls);
+        return launch_kernel(c, jk_row_entry(cp.X, cp.Y), cp.X, cp.Y, a, ls, 0);
+      }
+      for (int part = 0; part < (split ? 2 : 1); ++part) {
+        a.mode = split ? 1 + part : 0;
+        // the FP32 half reads the low-degree Boys table
+        a.boys = c->d_boys + ((split && part == 1) ? boys_low_offset(Lq) : (size_t)Lq * kBoysTableDoubles);
+        a.counters = counters();
+        ++nlaunch_class;
+        ++launches;
+        const int r = launch_class(c, cp.X, cp.Y, a, ls, split && part == 1 ? 1 : 0, cp.bucket == 0);
+        if (r) return r;
+      }
+      return DGF_OK;
+    };
+    // Clears the accumulators on `ls`, then the launches, longest first over
+    // the forked streams, joined back to `ls`.
+    auto enqueue_all = [&](cudaStream_t ls) -> int {
+      DGF_CUDA_CHECK(cudaMemsetAsync(c->d_Fh, 0, ns * n2 * 8, ls));
+      DGF_CUDA_CHECK(cudaMemsetAsync(c->d_row_work, 0, (size_t)kRowSlots * kRowChunksMax * sizeof(unsigned), ls));
+      c->row_slot = 0;
+      if (c->profiling) {  // one after the other, so that each is timed by itself
+        for (const Item &it : items)
+          if (int r = enqueue(it, ls)) return r;
+        return DGF_OK;
+      }
+      std::vector<Item> ord(items);
+      std::stable_sort(ord.begin(), ord.end(), [](const Item &u, const Item &v) { return u.s > v.s; });
+      const int nf = (int)std::min<size_t>(kForkStreams, ord.size());
+      DGF_CUDA_CHECK(cudaEventRecord(c->ev_fork, ls));
+      for (int k = 1; k < nf; ++k) DGF_CUDA_CHECK(cudaStreamWaitEvent(c->fork[k], c->ev_fork, 0));
+      double load[kForkStreams] = {};
+      int r = DGF_OK;
+      for (const Item &it : ord) {
+        const int k = (int)(std::min_element(load, load + nf) - load);
+        load[k] += it.s;
+        r = enqueue(it, k == 0 ? ls : c->fork[k]);
+        if (r) break;
+      }
+      for (int k = 1; k < nf; ++k) {  // after a failed launch too: the streams' work ends before the caller's goes on
+        DGF_CUDA_CHECK(cudaEventRecord(c->ev_join[k], c->fork[k]));
+        DGF_CUDA_CHECK(cudaStreamWaitEvent(ls, c->ev_join[k], 0));
+      }
+      return r;
+    };
+    // Short builds are replayed as a graph from their second call on: the
+    // launches between the density transform and the epilogue depend on the
+    // plan and the options only, not on the caller's matrices.
+    dgf_graph *gr = nullptr;
+    if (seconds < kGraphSeconds && !c->profiling && nslot_total <= chunk) {
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+      if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+      if (cap == cudaStreamCaptureStatusNone) {
+        std::string key;
+        auto add = [&key](const auto &v) { key.append(reinterpret_cast<const char *>(&v), sizeof(v)); };
+        add(c->gen);
+        add(ns);
+        add(o.thrs);
+        add(a.dens_thr);
+        add(a.ice_thr);
+        add(a.icedif);
+        add(o.mixed_cutoff);
+        add(o.hfxmu);
+        add(o.shard_index);
+        add(o.shard_count);
+        add(stored);
+        add(count);
+        for (int s = 0; s < ns; ++s) {
+          add(slots[s0 + s].js);
+          add(slots[s0 + s].ks);
+          add(slots[s0 + s].ka);
+        }
+        gr = graph_entry(c, key);
+      }
+    }
+    int r = DGF_OK;
+    if (gr && gr->exec) {
+      launches += gr->launches;
+      DGF_CUDA_CHECK(cudaGraphLaunch(gr->exec, st));
+    } else if (gr && gr->seen > 1) {
+      const int64_t l0 = launches;
+      cudaGraph_t g = nullptr;
+      DGF_CUDA_CHECK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+      r = enqueue_all(c->stream);
+      cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+      if (!r && e == cudaSuccess) e = cudaGraphInstantiate(&gr->exec, g, 0);
+      if (g) cudaGraphDestroy(g);
+      if (r) return r;
+      if (e != cudaSuccess) gr->exec = nullptr;
+      DGF_CUDA_CHECK(e);
+      gr->launches = launches - l0;
+      DGF_CUDA_CHECK(cudaGraphLaunch(gr->exec, st));
+    } else {
+      r = enqueue_all(st);
+      if (r) return r;
     }
     // Combine the slots of this chunk into the outputs they belong to.
     for (int k = 0; k < ndmat; ++k) {
@@ -1289,7 +1749,7 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
     }
   }
   DGF_CUDA_CHECK(cudaGetLastError());
-  DGF_CUDA_CHECK(cudaEventRecord(c->ev1, st));
+  if (count) DGF_CUDA_CHECK(cudaEventRecord(c->ev1, st));
   st_code = finish_profile(c, st);
   if (st_code) return st_code;
   if (stats || c->profiling) {
@@ -1307,7 +1767,6 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
     if (!stats) return DGF_OK;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
-    (void)total_q;
     stats->quartets_total = (int64_t)(cnt[0] + cnt[2]);  // passed Schwarz: evaluated or density-skipped
     stats->quartets_fp64 = (int64_t)(cnt[0] - cnt[3]);
     stats->quartets_fp32 = (int64_t)cnt[3];
@@ -1317,6 +1776,21 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
     stats->ms_device = ms;
   }
   return DGF_OK;
+}
+
+// A direct build of c, in its resolved context where there is one.
+static int fock_direct(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double *dmat_dev, double *fmat_dev,
+                       const dgf_options *opt, cudaStream_t st, dgf_stats *stats) {
+  dgf_ctx *d = direct_ctx(c);
+  if (d == c) return fock_impl(c, ndmat, ifctyp, dmat_dev, fmat_dev, opt, st, stats);
+  dgf_options o;
+  dgf_default_options(&o);
+  if (opt) o = *opt;
+  o.thrs *= kPrimThrs;
+  d->profiling = c->profiling;
+  const int r = fock_impl(d, ndmat, ifctyp, dmat_dev, fmat_dev, &o, st, stats);
+  if (c->profiling) c->prof = d->prof;
+  return r;
 }
 
 static int check_fock_args(dgf_ctx *c, dgf_int ndmat, const dgf_int *ifctyp, const void *d, const void *f) {
@@ -1331,7 +1805,7 @@ extern "C" int dgf_fock_device(dgf_ctx *c, dgf_int ndmat, const dgf_int *ifctyp,
   int r = check_fock_args(c, ndmat, ifctyp, dmat_device, fmat_device);
   if (r || ndmat == 0) return r;
   DeviceGuard g(c->device);
-  return fock_impl(c, (int)ndmat, ifctyp, dmat_device, fmat_device, opt, (cudaStream_t)stream, stats);
+  return fock_direct(c, (int)ndmat, ifctyp, dmat_device, fmat_device, opt, (cudaStream_t)stream, stats);
 }
 
 // An integral kernel that writes whole blocks: the tuned choice unless it is
@@ -1365,6 +1839,7 @@ extern "C" int dgf_store_integrals(dgf_ctx *c, double thrs, int64_t max_bytes, v
   if (bytes) *bytes = tot * 8;
   if (max_bytes > 0 && tot * 8 > max_bytes)
     DGF_FAIL(DGF_ERR_NOMEM, "the integral store needs " + std::to_string(tot * 8) + " bytes, more than max_bytes");
+  ++c->gen;
   if (c->d_store) cudaFree(c->d_store);
   c->d_store = nullptr;
   c->store_doubles = 0;
@@ -1422,6 +1897,7 @@ extern "C" int dgf_store_integrals(dgf_ctx *c, double thrs, int64_t max_bytes, v
 extern "C" int dgf_store_release(dgf_ctx *c) {
   if (!c) DGF_FAIL(DGF_ERR_ARG, "ctx is NULL");
   DeviceGuard g(c->device);
+  ++c->gen;
   if (c->d_store) cudaFree(c->d_store);
   c->d_store = nullptr;
   c->store_doubles = 0;
@@ -1456,7 +1932,7 @@ extern "C" int dgf_fock(dgf_ctx *c, dgf_int ndmat, const dgf_int *ifctyp, const 
   }
   double *dD = c->d_io, *dF = c->d_io + ndmat * n2;
   DGF_CUDA_CHECK(cudaMemcpyAsync(dD, dmat, ndmat * n2 * 8, cudaMemcpyHostToDevice, c->stream));
-  r = fock_impl(c, (int)ndmat, ifctyp, dD, dF, opt, c->stream, stats);
+  r = fock_direct(c, (int)ndmat, ifctyp, dD, dF, opt, c->stream, stats);
   if (r) return r;
   DGF_CUDA_CHECK(cudaMemcpyAsync(fmat, dF, ndmat * n2 * 8, cudaMemcpyDeviceToHost, c->stream));
   DGF_CUDA_CHECK(cudaStreamSynchronize(c->stream));
@@ -1484,6 +1960,8 @@ extern "C" int dgf_copy_tuning(dgf_ctx *dst, const dgf_ctx *src) {
   if (!dst || !src) DGF_FAIL(DGF_ERR_ARG, "NULL context");
   memcpy(dst->choice, src->choice, sizeof(dst->choice));
   memcpy(dst->split_ok, src->split_ok, sizeof(dst->split_ok));
+  dst->user_tuned = src->user_tuned;
+  ++dst->gen;
   return DGF_OK;
 }
 
@@ -1496,9 +1974,13 @@ extern "C" int dgf_set_class_kernel(dgf_ctx *c, int la, int lb, int lc, int ld, 
   if (X < Y) std::swap(X, Y);
   const int p = precision == 32 ? 1 : 0;
   const bool bra1 = c->cls_max_npp[X] == 1;
-  if (!jk_kernel_variant(X, Y, p, variant, false, bra1).launch && !jk_kernel_variant(X, Y, p, variant, true, bra1).launch)
+  const bool row = p == 0 && bra1 && ((variant == kRowVariant && jk_row_entry(X, Y).launch) ||
+                                      (variant == kPackVariant && c->spherical && g_pack_table[X][Y].launch));
+  if (!row && !jk_kernel_variant(X, Y, p, variant, false, bra1).launch && !jk_kernel_variant(X, Y, p, variant, true, bra1).launch)
     DGF_FAIL(DGF_ERR_UNSUPPORTED, "no such kernel variant for this class and precision");
   c->choice[X][Y][p] = variant;
+  c->user_tuned = true;
+  ++c->gen;
   return DGF_OK;
 }
 
@@ -1528,6 +2010,9 @@ extern "C" int dgf_autotune(dgf_ctx *c, const double *dmat_device, const dgf_opt
   DGF_CUDA_CHECK(cudaEventCreate(&e0));
   DGF_CUDA_CHECK(cudaEventCreate(&e1));
   std::string rep = "[";
+  ++c->gen;
+  c->user_tuned = true;
+  c->row_slot = kRowSlots;  // the first row launch clears the task counters
   const int saved_prof = c->profiling;
   c->profiling = 0;
   // candidates are timed over all bucket entries of a class pair
@@ -1559,8 +2044,12 @@ extern "C" int dgf_autotune(dgf_ctx *c, const double *dmat_device, const dgf_opt
       // single-primitive launches, the cooperative kernels are not timed
       // (they are several times slower wherever both exist).
       const bool has_warp = bra1 && jk_kernel_variant(cp.X, cp.Y, p, -3, true, bra1).launch != nullptr;
-      for (int v = -4; v < kThreadVariants; ++v) {
-        if (!jk_kernel_variant(cp.X, cp.Y, p, v, false, bra1).launch &&
+      for (int v = kPackVariant; v < kThreadVariants; ++v) {
+        bool row = false;  // an entry of the class pair has a row (pack) kernel
+        for (size_t q = ip; q < jp; ++q)
+          row = row || (p == 0 && ((v == kRowVariant && row_ok(c, c->plan[q])) ||
+                                   (v == kPackVariant && pack_ok(c, c->plan[q]))));
+        if (!row && !jk_kernel_variant(cp.X, cp.Y, p, v, false, bra1).launch &&
             !jk_kernel_variant(cp.X, cp.Y, p, v, true, bra1).launch)
           continue;
         if (has_warp && (v == -1 || v == -2)) continue;
@@ -1579,9 +2068,18 @@ extern "C" int dgf_autotune(dgf_ctx *c, const double *dmat_device, const dgf_opt
             a.nquartet = cq.nquartet;
             // entries this candidate has no kernel for run the FP64 default (same for every candidate)
             const ClassKernel &kv = jk_kernel_variant(cq.X, cq.Y, p, v, cq.bucket == 0, bra1);
-            const ClassKernel &k = kv.launch ? kv : jk_kernel(cq.X, cq.Y, 0, cq.bucket == 0, bra1);
+            const bool rowq = row && (v == kRowVariant ? row_ok(c, cq) : pack_ok(c, cq));
+            if (rowq) set_row_args(c, cq, a, 0, cq.row_ntask);
+            if (rowq && v == kPackVariant) {
+              r = launch_pack(c, cq, a, st);
+              if (r) return r;
+              continue;
+            }
+            const ClassKernel &k = rowq ? jk_row_entry(cq.X, cq.Y)
+                                   : kv.launch ? kv
+                                               : jk_kernel(cq.X, cq.Y, 0, cq.bucket == 0, bra1);
             if (kv.launch) chunks = k.chunks;
-            r = launch_kernel(c, k, cq.X, cq.Y, a, st, kv.launch ? p : 0);
+            r = launch_kernel(c, k, cq.X, cq.Y, a, st, kv.launch ? p : 0);  // a row launch is FP64
             if (r) return r;
           }
           DGF_CUDA_CHECK(cudaEventRecord(e1, st));
@@ -1625,6 +2123,15 @@ extern "C" int dgf_autotune(dgf_ctx *c, const double *dmat_device, const dgf_opt
             a.split = o.mixed_cutoff;
             // as in the build: entries without an FP32 kernel are not split
             const bool cansplit = select_kernel(c, cq.X, cq.Y, 1, cq.bucket == 0).launch != nullptr;
+            const int route = class_route(c, cq, 1, false);
+            if (!(cfg && cansplit) && route != kRouteOther) {
+              set_row_args(c, cq, a, 0, cq.row_ntask);
+              a.mode = 0;
+              r = route == kRoutePack ? launch_pack(c, cq, a, st)
+                                      : launch_kernel(c, jk_row_entry(cq.X, cq.Y), cq.X, cq.Y, a, st, 0);
+              if (r) return r;
+              continue;
+            }
             for (int part = 0; part < (cfg && cansplit ? 2 : 1); ++part) {
               const int prec = (cfg && part == 1) ? 1 : 0;
               a.mode = (cfg && cansplit) ? 1 + part : 0;
@@ -1640,10 +2147,10 @@ extern "C" int dgf_autotune(dgf_ctx *c, const double *dmat_device, const dgf_opt
       }
       a.dmax = nullptr;
       a.mode = 0;
-      c->split_ok[cp.X][cp.Y] = t[1] < t[0] ? 1 : 0;
+      c->split_ok[cp.X][cp.Y] = t[1] < t[0] ? 2 : 0;
       char buf[160];
       snprintf(buf, sizeof(buf), "%s{\"class\":[%d,%d,%d,%d],\"split\":%d,\"ms_fp64\":%.4f,\"ms_split\":%.4f}",
-               rep.size() > 1 ? "," : "", la, lb, lc, ld, c->split_ok[cp.X][cp.Y], t[0], t[1]);
+               rep.size() > 1 ? "," : "", la, lb, lc, ld, c->split_ok[cp.X][cp.Y] ? 1 : 0, t[0], t[1]);
       rep += buf;
     }
     ip = jp;

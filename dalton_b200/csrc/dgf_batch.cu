@@ -30,6 +30,8 @@ struct BatchPlan {
   int64_t off;       // into the qoff buffer (nbra+1 entries)
   int64_t koff;      // into the kbase buffer (nbra entries)
   int64_t nquartet;
+  int64_t row_off = 0;  // row kernel: its tasks (row_ntask 0: none)
+  int row_ntask = 0;
 };
 
 struct dgf_batch {
@@ -39,6 +41,16 @@ struct dgf_batch {
   std::vector<int> nbf, nwf;
   int64_t total = 0, total_w = 0;
   std::vector<PairRec> pairs;
+  // row kernels: the bras of every class in row order, molecule by molecule
+  // (positions in the merged class list), the ket table of single-primitive
+  // kets, fine Boys tables, the plan's tasks and the launches' task counters
+  std::vector<int> row_bra;
+  int *d_row_bra = nullptr;
+  int4 *d_ks_i = nullptr;
+  double *d_ks_q = nullptr, *d_ks_pp = nullptr, *d_fine = nullptr;
+  int4 *d_row_tasks = nullptr;
+  unsigned *d_row_work = nullptr;
+  double thrs_scale = 1.0;  // of the caller's Schwarz threshold (resolved contexts)
   int cls_off[kNumPairClass + 1] = {0};
   std::vector<int> mol_cls_off;  // [X * nmol + m]: start of molecule m's class-X pairs in the merged list
   std::vector<int> mol_bkt;      // [(X * nmol + m) * (kNumBuckets + 1) + k]: bucket starts inside that list
@@ -93,7 +105,8 @@ static void batch_free(dgf_batch *b) {
   if (b->graph) cudaGraphDestroy(b->graph);
   void *ptrs[] = {b->d_pairs, b->d_pp,  b->d_boys, b->d_sph,  b->d_offsets, b->d_dims,  b->d_wmap_i,
                   b->d_wmap_c, b->d_D,   b->d_Ds,   b->d_Fh,   b->d_cnt,     b->d_qoff,  b->d_kbase,
-                  b->d_bsh,    b->d_bmol, b->d_bpref, b->d_dmw};
+                  b->d_bsh,    b->d_bmol, b->d_bpref, b->d_dmw,   b->d_row_bra, b->d_ks_i,  b->d_ks_q,
+                  b->d_ks_pp,  b->d_fine, b->d_row_tasks, b->d_row_work};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -115,12 +128,24 @@ static void batch_free(dgf_batch *b) {
 
 extern "C" void dgf_batch_destroy(dgf_batch *b) { batch_free(b); }
 
-extern "C" int dgf_batch_create(dgf_ctx *const *ctxs, dgf_int nmol, dgf_batch **out) {
+extern "C" int dgf_batch_create(dgf_ctx *const *caller_ctxs, dgf_int nmol, dgf_batch **out) {
   if (!out) BFAIL(DGF_ERR_ARG, "out is NULL");
   *out = nullptr;
-  if (!ctxs || nmol <= 0) BFAIL(DGF_ERR_ARG, "empty batch");
+  if (!caller_ctxs || nmol <= 0) BFAIL(DGF_ERR_ARG, "empty batch");
   for (dgf_int m = 0; m < nmol; ++m)
-    if (!ctxs[m]) BFAIL(DGF_ERR_ARG, "NULL context in batch");
+    if (!caller_ctxs[m]) BFAIL(DGF_ERR_ARG, "NULL context in batch");
+  // Contracted contexts take part in their resolved form where all of them
+  // have it (one tuned context keeps the batch contracted: its choices are
+  // for the contracted classes).
+  std::vector<dgf_ctx *> ctxs(caller_ctxs, caller_ctxs + nmol);
+  bool tuned = false, resolved = false;
+  for (dgf_ctx *c : ctxs) tuned = tuned || c->user_tuned;
+  if (!tuned)
+    for (dgf_ctx *&c : ctxs) {
+      dgf_ctx *d = direct_ctx(c);
+      resolved = resolved || d != c;
+      c = d;
+    }
   const int dev = ctxs[0]->device, sph = ctxs[0]->spherical;
   for (dgf_int m = 0; m < nmol; ++m)
     if (ctxs[m]->device != dev || ctxs[m]->spherical != sph)
@@ -130,6 +155,7 @@ extern "C" int dgf_batch_create(dgf_ctx *const *ctxs, dgf_int nmol, dgf_batch **
   b->nmol = (int)nmol;
   b->spherical = sph;
   b->nsm = ctxs[0]->nsm;
+  b->thrs_scale = resolved ? kPrimThrs : 1.0;
   DeviceGuard g(dev);
   b->offsets.assign(nmol + 1, 0);
   b->woffsets.assign(nmol + 1, 0);
@@ -191,6 +217,8 @@ extern "C" int dgf_batch_create(dgf_ctx *const *ctxs, dgf_int nmol, dgf_batch **
     b->cls_off[X] = (int)b->pairs.size();
     for (dgf_int m = 0; m < nmol; ++m) {
       const dgf_ctx *c = ctxs[m];
+      for (int i = c->cls_off[X]; i < c->cls_off[X + 1]; ++i)
+        b->row_bra.push_back(c->row_bra[i] + (int)b->pairs.size() - b->cls_off[X]);
       b->mol_cls_off[(size_t)X * nmol + m] = (int)b->pairs.size();
       // The molecule's class list in its context's order: primitive-count
       // bucket, Schwarz bin, shells (a bra's partners in one bucket are a
@@ -244,6 +272,24 @@ extern "C" int dgf_batch_create(dgf_ctx *const *ctxs, dgf_int nmol, dgf_batch **
   alloc((void **)&b->d_Ds, b->total_w * 8);
   alloc((void **)&b->d_Fh, b->total_w * 8);
   alloc((void **)&b->d_cnt, 4 * kCounterSlots * 8);
+  const size_t npair = b->pairs.size();
+  std::vector<int4> ki(npair);
+  std::vector<double> kq(npair), kp(11 * npair);
+  for (size_t i = 0; i < npair; ++i) {
+    const PairRec &r = b->pairs[i];
+    ki[i] = make_int4(r.aoA, r.aoB, r.same, 0);
+    kq[i] = r.Q;
+    const PrimPair &q = pp[r.pp0];
+    const double v[11] = {q.p, q.Px, q.Py, q.Pz, q.K, q.PAx, q.PAy, q.PAz, q.PBx, q.PBy, q.PBz};
+    for (int k = 0; k < 11; ++k) kp[k * npair + i] = v[k];
+  }
+  const size_t n_fine = (size_t)(kFineMaxM + 1) * kFineDoubles;
+  alloc((void **)&b->d_row_bra, npair * 4);
+  alloc((void **)&b->d_ks_i, npair * sizeof(int4));
+  alloc((void **)&b->d_ks_q, npair * 8);
+  alloc((void **)&b->d_ks_pp, 11 * npair * 8);
+  alloc((void **)&b->d_fine, n_fine * 8);
+  alloc((void **)&b->d_row_work, (size_t)kRowSlots * kRowChunksMax * sizeof(unsigned));
   alloc((void **)&b->d_bsh, bsh.size() * 4);
   alloc((void **)&b->d_bmol, bmol.size() * 4);
   alloc((void **)&b->d_bpref, bpref.size() * 8);
@@ -260,6 +306,11 @@ extern "C" int dgf_batch_create(dgf_ctx *const *ctxs, dgf_int nmol, dgf_batch **
   if (e == cudaSuccess) e = cudaMemcpy(b->d_dims, dims.data(), dims.size() * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->d_wmap_i, ints.data(), ints.size() * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && !cs.empty()) e = cudaMemcpy(b->d_wmap_c, cs.data(), cs.size() * 8, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && npair) e = cudaMemcpy(b->d_row_bra, b->row_bra.data(), npair * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && npair) e = cudaMemcpy(b->d_ks_i, ki.data(), npair * sizeof(int4), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && npair) e = cudaMemcpy(b->d_ks_q, kq.data(), npair * 8, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && npair) e = cudaMemcpy(b->d_ks_pp, kp.data(), 11 * npair * 8, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(b->d_fine, ctxs[0]->d_fine, n_fine * 8, cudaMemcpyDeviceToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->d_bsh, bsh.data(), bsh.size() * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->d_bmol, bmol.data(), bmol.size() * 4, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->d_bpref, bpref.data(), bpref.size() * 8, cudaMemcpyHostToDevice);
@@ -308,6 +359,7 @@ static int batch_plan(dgf_batch *b, double thrs) {
   std::vector<int64_t> qoff;
   std::vector<int> kbase;
   std::vector<BatchPlan> plan;
+  std::vector<int4> tasks;
   const int nm = b->nmol;
   auto mol_end = [&](int X, int m) {
     return (m + 1 < nm) ? b->mol_cls_off[(size_t)X * nm + m + 1] : b->cls_off[X + 1];
@@ -350,6 +402,24 @@ static int batch_plan(dgf_batch *b, double thrs) {
           }
         }
         bp.nquartet = acc;
+        // Row kernel, as for one molecule: single-primitive pairs, spherical
+        // functions, 32-bit offsets within a molecule's matrices.
+        const bool sph = b->spherical || (X < 3 && Y < 3);
+        const int nwmax = *std::max_element(b->nwf.begin(), b->nwf.end());
+        if (acc > 0 && kb == 0 && b->cls_max_npp[X] == 1 && sph && nwmax <= 46340 && jk_row_entry(X, Y).launch) {
+          std::vector<RowSource> src;
+          for (int m = 0; m < nm; ++m) {
+            const int b0 = b->mol_cls_off[(size_t)X * nm + m] - b->cls_off[X], nbm = mol_end(X, m) - b->cls_off[X] - b0;
+            const int ky = b->mol_cls_off[(size_t)Y * nm + m] - b->cls_off[Y];
+            const int *bk = &b->mol_bkt[((size_t)Y * nm + m) * (kNumBuckets + 1)];
+            if (nbm > 0 && bk[kb + 1] > bk[kb])
+              src.push_back(RowSource{b->row_bra.data() + b->cls_off[X] + b0, nbm, &b->pairs[b->cls_off[X]],
+                                      &qoff[bp.off], b0, ky + bk[kb], ky + bk[kb + 1]});
+          }
+          bp.row_off = (int64_t)tasks.size();
+          row_tasks(src, row_max_bras(X), 32, tasks);
+          bp.row_ntask = (int)(tasks.size() - bp.row_off);
+        }
         if (acc > 0)
           plan.push_back(bp);
         else {
@@ -359,8 +429,19 @@ static int batch_plan(dgf_batch *b, double thrs) {
       }
   if (b->d_qoff) cudaFree(b->d_qoff);
   if (b->d_kbase) cudaFree(b->d_kbase);
+  if (b->d_row_tasks) cudaFree(b->d_row_tasks);
   b->d_qoff = nullptr;
   b->d_kbase = nullptr;
+  b->d_row_tasks = nullptr;
+  if (!tasks.empty()) {
+    if (cudaMalloc(&b->d_row_tasks, tasks.size() * sizeof(int4)) != cudaSuccess) {
+      cudaGetLastError();
+      b->plan.clear();
+      BFAIL(DGF_ERR_NOMEM, "device allocation of the batch plan failed");
+    }
+    if (cudaMemcpy(b->d_row_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess)
+      BFAIL(DGF_ERR_CUDA, "upload of the batch plan failed");
+  }
   if (cudaMalloc(&b->d_qoff, std::max<size_t>(qoff.size(), 1) * 8) != cudaSuccess ||
       cudaMalloc(&b->d_kbase, std::max<size_t>(kbase.size(), 1) * 4) != cudaSuccess) {
     cudaGetLastError();
@@ -429,7 +510,9 @@ static int batch_enqueue(dgf_batch *b, const double *din, double *fout, double h
                                              b->nshell_all, b->nmol, b->nshpair, b->d_dmw);
     ++launches;
   }
-  if (cudaMemsetAsync(b->d_Fh, 0, b->total_w * 8, st) != cudaSuccess) BFAIL(DGF_ERR_CUDA, "memset failed");
+  if (cudaMemsetAsync(b->d_Fh, 0, b->total_w * 8, st) != cudaSuccess ||
+      cudaMemsetAsync(b->d_row_work, 0, (size_t)kRowSlots * kRowChunksMax * sizeof(unsigned), st) != cudaSuccess)
+    BFAIL(DGF_ERR_CUDA, "memset failed");
   JKArgs a;
   memset(&a, 0, sizeof(a));
   a.pp = b->d_pp;
@@ -471,7 +554,7 @@ static int batch_enqueue(dgf_batch *b, const double *din, double *fout, double h
   if (cudaEventRecord(b->ev_fork, st) != cudaSuccess) BFAIL(DGF_ERR_CUDA, "event record failed");
   for (int k = 0; k < ns; ++k)
     if (cudaStreamWaitEvent(b->aux[k], b->ev_fork, 0) != cudaSuccess) BFAIL(DGF_ERR_CUDA, "stream fork failed");
-  int slot = 0;
+  int slot = 0, row_slot = 0;
   for (int i : order) {
     const BatchPlan &bp = b->plan[i];
     cudaStream_t ls = b->aux[stream_of[i]];
@@ -492,6 +575,33 @@ static int batch_enqueue(dgf_batch *b, const double *din, double *fout, double h
     // for quartets whose bound is at or above the cutoff and an FP32 launch
     // for the rest.
     const ClassKernel *k32 = nullptr;
+    const int choice = b->choice[bp.X][bp.Y];
+    const bool row = bp.row_ntask > 0 && row_slot < kRowSlots && (choice == kDefaultVariant || choice == kRowVariant) &&
+                     !(mixed && b->split_ok[bp.X][bp.Y] == 2);
+    if (row) {
+      const ClassKernel &k = jk_row_entry(bp.X, bp.Y);
+      a.mode = 0;
+      a.counters = b->d_cnt + 4 * (slot++ % kCounterSlots);
+      a.boys_fine = b->d_fine + (size_t)Lq * kFineDoubles;
+      a.ks_i = b->d_ks_i;
+      a.ks_q = b->d_ks_q;
+      a.ks_pp = b->d_ks_pp;
+      a.ks_stride = (int64_t)b->pairs.size();
+      a.ks_base = b->cls_off[bp.Y];
+      a.row_bra = b->d_row_bra + b->cls_off[bp.X];
+      a.row_tasks = b->d_row_tasks + bp.row_off;
+      a.row_task0 = 0;
+      a.row_task1 = bp.row_ntask;
+      a.row_work = b->d_row_work + (size_t)kRowChunksMax * row_slot++;
+      const int warps = k.block / 32;
+      k.launch(a, std::max(1, std::min((bp.row_ntask + warps - 1) / warps, (b->nsm * k.qpb + k.chunks - 1) / k.chunks)),
+               k.block, k.smem, ls);
+      a.ks_i = nullptr;  // the other kernels read the records: their kets are not one adjacent run
+      a.ks_q = nullptr;
+      a.ks_pp = nullptr;
+      ++launches;
+      continue;
+    }
     if (mixed && b->split_ok[bp.X][bp.Y]) {
       k32 = &jk_kernel_variant(bp.X, bp.Y, 1, b->choice32[bp.X][bp.Y], bp.bucket == 0, bra1);
       if (!k32->launch) k32 = &jk_kernel(bp.X, bp.Y, 1, bp.bucket == 0, bra1);
@@ -538,6 +648,7 @@ extern "C" int dgf_fock_batch(dgf_batch *b, const double *dmat_packed_device, do
     }
   }
   cudaStream_t st = (cudaStream_t)stream;  // NULL: the legacy default stream, as in dgf_fock_device
+  o.thrs *= b->thrs_scale;
   int r = batch_plan(b, o.thrs);
   if (r) return r;
   if (cudaMemsetAsync(b->d_cnt, 0, 4 * kCounterSlots * 8, st) != cudaSuccess) BFAIL(DGF_ERR_CUDA, "memset failed");

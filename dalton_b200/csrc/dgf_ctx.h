@@ -24,7 +24,12 @@ struct ClassPlan {
   int kb0, kb1;       // ket range of this entry: one primitive-count bucket of class Y (relative to its start)
   int64_t off;        // offset of this entry's qoff array in the plan buffer
   int64_t nquartet;
+  // row kernels, Fock and gradient (row_ntask 0: none): their tasks in d_row_tasks
+  int64_t row_off = 0;
+  int row_ntask = 0;
 };
+// Task counters of the row launches of a call (kRowChunksMax each).
+constexpr int kRowSlots = 128;
 
 // Map between the AO basis (Dalton's contracted functions) and the
 // two-electron working basis, as sparse rows: wr_* gives, for every working
@@ -34,6 +39,20 @@ struct ClassPlan {
 struct WorkMapHost {
   std::vector<int> wr_off, wr_idx, ac_off, ac_idx;
   std::vector<double> wr_c, ac_c;
+};
+
+// Streams the class launches of a build are spread over (the caller's is the
+// first), so that the tail of one launch, or a launch too small to fill the
+// GPU, runs beside others.
+constexpr int kForkStreams = 8;
+
+// A build captured as a graph (fock_impl): its options, the executable graph
+// (null before the second call), kernel launches in it, calls seen.
+struct dgf_graph {
+  std::string key;
+  cudaGraphExec_t exec;
+  int64_t launches;
+  int64_t seen;
 };
 
 struct dgf_ctx {
@@ -48,6 +67,18 @@ struct dgf_ctx {
   // primitive; every other block keeps one shell per contracted function.
   // nwf functions in nwshell shells; w_identity when no block was resolved
   // (the working basis is then the AO basis, function for function).
+  // A context whose blocks are segmented contractions (several primitives,
+  // none shared) keeps them contracted; `prim` is then a second context with
+  // every contracted shell resolved into its primitives, which direct Fock
+  // builds and gradients use (direct_ctx).  It is made by the first of them
+  // from the copy of the basis kept here.
+  bool resolve_all = false;   // this is such a second context
+  bool prim_fits = false;     // the resolved form exists and fits every entry point
+  bool user_tuned = false;    // kernel choices were made for this context: it serves all calls itself
+  dgf_ctx *prim = nullptr;
+  dgf_basis basis_copy = {};
+  std::vector<dgf_int> basis_i;
+  std::vector<double> basis_d;
   int nwf = 0, nwshell = 0, w_identity = 1;
   std::vector<int> ws_l, ws_atom, ws_ao, ws_nprim, ws_p0;
   std::vector<double> ws_a, ws_c;
@@ -56,6 +87,8 @@ struct dgf_ctx {
   double *d_wmap_c = nullptr;   // wr_c | ac_c
   int64_t *d_wmeta = nullptr;   // {0, nwf^2} {0, nbf^2} element offsets of the single-molecule form
   int *d_wdims = nullptr;       // {nwf, nbf, 0, 0}
+  double *d_one = nullptr;      // scratch of the one-electron calls (dgf_grad.cu), made by the first of them
+  double *d_pg = nullptr;       // two-electron gradient: derivatives per pair (6 each), then task counters
   double *d_gw = nullptr;       // working-basis densities of the two-electron gradient (2 nwf^2)
   int *d_shinfo = nullptr;      // per working shell: first function | function count (density bounds)
   // conventional form: the integral store (dgf_store_integrals) for the plan
@@ -79,6 +112,17 @@ struct dgf_ctx {
   double *d_ks_q = nullptr, *d_ks_pp = nullptr;
   dgf::PrimPair *d_pp = nullptr;
   double *d_boys = nullptr, *d_sph = nullptr;
+  // row kernels: fine Boys tables, bra pairs in row order (by class, A shell,
+  // primitive-count bucket, Schwarz factor descending; positions within the
+  // class), the plan's tasks and the launches' task counters
+  double *d_fine = nullptr;
+  std::vector<int> row_bra;
+  int *d_row_bra = nullptr;
+  int4 *d_row_tasks = nullptr;
+  size_t row_tasks_cap = 0;
+  double *d_frag[dgf::kNumPairClass] = {};  // pack kernels: the classes' pair fragments, made with the first plan that uses them
+  unsigned *d_row_work = nullptr;
+  int row_slot = 0;  // next free slot of d_row_work in the running call
   // per-call buffers
   int cap_slots = 0, cap_io = 0;
   double *d_D = nullptr, *d_Ds = nullptr, *d_Fh = nullptr, *d_io = nullptr;
@@ -102,12 +146,18 @@ struct dgf_ctx {
   size_t qoff_cap = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  // kernel choice per class pair and precision (-1 = team kernel, >= 0 =
-  // thread-kernel variant), set by the autotuner; 0 by default
+  cudaStream_t fork[kForkStreams] = {};
+  cudaEvent_t ev_fork = nullptr, ev_join[kForkStreams] = {};
+  std::vector<dgf_graph> graphs;
+  int64_t gen = 0, graph_gen = 0;  // counts changes of plan, buffers and kernel choices; of the kept graphs
+  // kernel choice per class pair and precision (-5 = row kernel, -1 = team
+  // kernel, >= 0 = thread-kernel variant), set by the autotuner;
+  // kDefaultVariant by default
   int choice[dgf::kNumPairClass][dgf::kNumPairClass][2] = {};
   // mixed form: whether a class pair is split into FP64 and FP32 launches
-  // (set by the autotuner where the FP32 half pays for the second pass over
-  // the class's quartets; every class splits by default)
+  // (1: by default, where the class has no row kernel; set by the autotuner
+  // to 2 where the FP32 half pays for the second pass over the class's
+  // quartets, to 0 elsewhere)
   int split_ok[dgf::kNumPairClass][dgf::kNumPairClass];
   // per-class launch profiling (dgf_set_profiling)
   int profiling = 0;
@@ -115,6 +165,28 @@ struct dgf_ctx {
   std::vector<dgf_class_time> prof;
 };
 
+// Bra pairs of one molecule and class for row_tasks: their row order (class
+// positions), the class list, the plan's prefix sums by class position, the
+// place of the first one in the launch's row_bra list, and their kets.
+struct RowSource {
+  const int *order;
+  int n;
+  const dgf::PairRec *pairs;
+  const int64_t *qoff;
+  int bra0, ket0, ket_end;
+};
+// Appends the row tasks of a launch (dgf_api.cu).
+void row_tasks(const std::vector<RowSource> &src, int max_bras, int min_width, std::vector<int4> &tasks);
+
+// Schwarz threshold of a resolved context for the caller's threshold: a
+// contracted integral is a sum of primitive ones, so the primitives are
+// screened more tightly than the contracted quartet would be.  At the same
+// threshold the Fock matrix of H2O / 6-31G* was 2e-13 from the unscreened
+// one (relative), where the contracted form drops nothing.
+constexpr double kPrimThrs = 1e-3;
+// The context a direct build or gradient of `c` runs in: its resolved form
+// when it has one and nothing was tuned on `c`, else itself (dgf_api.cu).
+dgf_ctx *direct_ctx(dgf_ctx *c);
 
 // The single-molecule form of the AO <-> working-basis maps of a context.
 inline dgf::WorkMaps ctx_maps(const dgf_ctx *c) {

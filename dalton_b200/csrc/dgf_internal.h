@@ -57,6 +57,17 @@ __host__ __device__ constexpr size_t boys_low_offset(int M) {
   return ((size_t)(kBoysMaxM + 1) + M) * kBoysTableDoubles;
 }
 
+// Fine table of the row kernels: F_M on the same range in intervals of
+// 1/kFinePerUnit, degree 7, one row of kFineStride doubles per interval:
+// eight coefficients, e^-mid, one unused (rows stay 16-byte aligned, and 80
+// bytes apart they spread over all shared-memory banks).
+constexpr int kFinePerUnit = 8;
+constexpr int kFineDeg = 7;
+constexpr int kFineStride = 10;
+constexpr int kFineNint = 320;
+constexpr int kFineDoubles = kFineNint * kFineStride;
+constexpr int kFineMaxM = 6;  // orders 0 .. kFineMaxM
+
 __host__ __device__ constexpr int ncart(int l) { return (l + 1) * (l + 2) / 2; }
 __host__ __device__ constexpr int n3(int L) { return (L + 1) * (L + 2) * (L + 3) / 6; }
 __host__ __device__ constexpr int pair_class(int la, int lb) { return la * (la + 1) / 2 + lb; }
@@ -158,6 +169,15 @@ struct JKArgs {
   const double *ks_pp;
   int64_t ks_stride;
   int ks_base;
+  // row kernels (dgf_jk_row.cuh): the fine Boys table of order L, the bra
+  // pairs in row order (class-relative positions), the tasks {first bra,
+  // bras, first 32-ket chunk, chunks} of this launch, the kets of the plan
+  // entry, and the task counters (one per A chunk, zero at the launch)
+  const double *boys_fine;
+  const int *row_bra;
+  const int4 *row_tasks;
+  unsigned *row_work;
+  int row_task0, row_task1, row_nket;
   // gradient mode (dgf_grad2e): densities D1, D2 (N*N) and grad (natom*3)
   const double *G1, *G2;
   double *grad;
@@ -176,18 +196,23 @@ constexpr int kSphTableDoubles = 1 * 1 + 3 * 3 + 5 * 6 + 7 * 10 + 9 * 15;
 
 typedef void (*JKLauncher)(const JKArgs &, int grid, int block, size_t smem, cudaStream_t);
 
-enum { kKindThread = 0, kKindTeam = 1, kKindWarpTeam = 2, kKindWarp = 4, kKindWarpMma = 6 };
+enum { kKindThread = 0, kKindTeam = 1, kKindWarpTeam = 2, kKindWarp = 4, kKindWarpMma = 6, kKindRow = 8 };
 
 struct ClassKernel {
   JKLauncher launch;
   int block;
-  size_t smem;   // dynamic shared memory (team and warp kernels); 0 for thread kernels
-  int chunks;    // thread kernels: A-component chunks (grid.y)
-  int qpb;       // quartets a block works on at a time (grid sizing)
-  int kind;      // kKindThread, kKindTeam, kKindWarpTeam, kKindWarp or kKindWarpMma
+  size_t smem;   // dynamic shared memory (team, warp and row kernels); 0 for thread kernels
+  int chunks;    // thread and row kernels: A-component chunks (grid.y)
+  int qpb;       // quartets a block works on at a time (grid sizing); row kernels: resident blocks per SM
+  int kind;      // kKindThread, kKindTeam, kKindWarpTeam, kKindWarp, kKindWarpMma or kKindRow
 };
 
 constexpr int kThreadVariants = 2;
+constexpr int kRowVariant = -5;        // the row kernel (single-primitive pairs, one density slot)
+constexpr int kDefaultVariant = -100;  // no choice made: the class's default kernel
+// Most bras of a row-kernel segment of bra class X (staged in shared memory).
+__host__ __device__ constexpr int row_max_bras(int X) { return X == 0 ? 32 : 16; }
+constexpr int kRowChunksMax = 8;  // A chunks of a row kernel at most (task counters per launch)
 
 // Per-class launch table (filled by dgf_jk.cu): index [X][Y] of pair classes.
 // precision: 0 = default FP64 kernel, 1 = FP32 kernel, 2 = team kernel.
@@ -201,9 +226,13 @@ const ClassKernel &jk_stored_kernel(int X, int Y);
 // kernel, >= 0 = thread-kernel variant (precision 0/1).
 const ClassKernel &jk_kernel_variant(int X, int Y, int precision, int variant, bool ket1 = false,
                                      bool bra1 = false);
+// Row kernel of class pair (X, Y) (launch null: none).  Its launches take the
+// tasks of a plan entry (JKArgs::row_*).
+const ClassKernel &jk_row_entry(int X, int Y);
 cudaError_t jk_prepare_all();
 
 void boys_table_host(std::vector<double> &out);       // [kBoysMaxM+1][kBoysTableDoubles]
+void boys_fine_host(std::vector<double> &out);        // [kFineMaxM+1][kFineDoubles]
 void sph_table_host(std::vector<double> &out);        // kSphTableDoubles
 double boys_reference(int m, double t);               // accurate host F_m(t)
 

@@ -5,10 +5,14 @@
 // A-chunk variants (the per-class tuning space).  The entries are filled by
 // generated translation units (dgf_jk_inst.cuh).
 #include "dgf_jk_inst.cuh"
+#include "dgf_pack.h"
 
 namespace dgf {
 
 JKEntry g_jk_table[kNumPairClass][kNumPairClass];
+PackEntry g_pack_table[kNumPairClass][kNumPairClass];
+FragEntry g_frag_table[kNumPairClass];
+ClassKernel g_row_stored[kNumPairClass][kNumPairClass];
 
 namespace {
 const ClassKernel kNone{nullptr, 0, 0, 0, 0, 0};
@@ -23,6 +27,7 @@ const ClassKernel kNone{nullptr, 0, 0, 0, 0, 0};
 const ClassKernel &jk_kernel_variant(int X, int Y, int precision, int variant, bool ket1, bool bra1) {
   const JKEntry &e = g_jk_table[X][Y];
   const int p = precision ? 1 : 0;
+  if (variant < -4) return kNone;  // row kernels need a plan's tasks: jk_row_entry
   if (variant == -4) return precision == 0 ? e.warp_mma : kNone;
   if (variant == -3) return ((ket1 && bra1) || e.warp_mp) ? e.warp[p] : kNone;
   if (variant == -2) return precision == 0 ? e.wteam : kNone;
@@ -44,14 +49,17 @@ const ClassKernel &jk_kernel(int X, int Y, int precision, bool ket1, bool bra1) 
   return precision == 1 ? kNone : e.team;
 }
 
+const ClassKernel &jk_row_entry(int X, int Y) { return g_jk_table[X][Y].row; }
+
 const ClassKernel &jk_stored_kernel(int X, int Y) { return g_jk_table[X][Y].stored; }
 
 cudaError_t jk_prepare_all() {
   for (int X = 0; X < kNumPairClass; ++X)
     for (int Y = 0; Y <= X; ++Y)
-      for (int P = 0; P < 3; ++P) {
+      for (int P = 0; P < 4; ++P) {
         if (!g_jk_table[X][Y].prepare[P]) return cudaErrorInitializationError;  // a generated part is missing
         cudaError_t e = g_jk_table[X][Y].prepare[P]();
+        if (e == cudaSuccess && P == 0 && g_pack_table[X][Y].prepare) e = g_pack_table[X][Y].prepare();
         if (e != cudaSuccess) return e;
       }
   return cudaSuccess;

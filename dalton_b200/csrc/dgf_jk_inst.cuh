@@ -1,10 +1,10 @@
 // The quartet-class kernel table of libdgfock and what its instantiation
-// units share.  The entry of class pair (X, Y) is filled by three generated
+// units share.  The entry of class pair (X, Y) is filled by four generated
 // translation units (parts) so that the heaviest classes compile in
 // parallel and a change to one kernel family rebuilds only its units:
 // part 0 the cooperative, warp-team and warp-per-quartet kernels
 // (dgf_jk_inst_team.cuh), parts 1 and 2 the FP64 and FP32 thread kernels
-// (dgf_jk_inst_thread.cuh).  Each part sets only its own fields of the
+// (dgf_jk_inst_thread.cuh), part 3 the row kernel (dgf_jk_inst_row.cuh).  Each part sets only its own fields of the
 // (zero-initialised) entry and its own prepare hook.
 #pragma once
 
@@ -21,7 +21,8 @@ struct JKEntry {
   bool warp_mp;                          // the warp kernel loops over primitive pairs (else one per side only)
   ClassKernel warp_mma;                  // warp-per-quartet kernel with DMMA transforms (FP64, any pairs)
   ClassKernel stored;                    // digestion of stored integral blocks (conventional form)
-  cudaError_t (*prepare[3])();           // one per generated part
+  ClassKernel row;                       // row kernel (single-primitive pairs, spherical functions, one density slot)
+  cudaError_t (*prepare[4])();           // one per generated part
 };
 
 extern JKEntry g_jk_table[kNumPairClass][kNumPairClass];

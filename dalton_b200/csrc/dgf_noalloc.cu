@@ -78,6 +78,10 @@ extern "C" int dgf_fock_device_noalloc(dgf_ctx *c, const double *dmat_device, do
     return fail(DGF_ERR_ARG, __LINE__,
                 "dgf_fock_device_noalloc: " + std::to_string(c->nbf) + " basis functions exceed its fixed scratch (" +
                     std::to_string(kNoAllocMaxN) + " at most); use dgf_fock_device");
+  if (c->prim && direct_ctx(c) == c->prim) {  // where the caller's dgf_fock calls made their plan
+    c = c->prim;
+    thrs *= kPrimThrs;
+  }
   if (c->nwf > kNoAllocMaxW)
     return fail(DGF_ERR_ARG, __LINE__,
                 "dgf_fock_device_noalloc: " + std::to_string(c->nwf) + " working functions exceed its fixed scratch (" +

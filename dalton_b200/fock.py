@@ -80,7 +80,7 @@ class FockBuilder:
 
     def set_class_kernel(self, cls, variant, precision=64):
         """Pin the kernel of quartet class ``cls`` = (la, lb, lc, ld): variant
-        -4 warp per quartet with FP64 tensor-core (DMMA) transforms, -3 warp
+        -5 row kernel (FP64), -4 warp per quartet with FP64 tensor-core (DMMA) transforms, -3 warp
         per quartet, -2 warp team, -1 cooperative team, 0.. thread chunk
         variants."""
         la, lb, lc, ld = (int(x) for x in cls)

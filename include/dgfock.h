@@ -210,7 +210,8 @@ typedef struct {
   int32_t precision;        /* 64 = FP64, 32 = FP32 contraction */
   int32_t kernel;           /* 0 = thread-per-quartet, 1 = cooperative team, 2 = warp teams,
                                4 = warp-per-quartet (L >= 4), 6 = warp-per-quartet with
-                               FP64 tensor-core (DMMA) transforms,
+                               FP64 tensor-core (DMMA) transforms, 8 = row kernel (a warp on
+                               bra pairs of one A shell times 32 kets),
                                5 = two-electron gradient (dgf_grad2e*: quartets are the plan's,
                                primitive quartets estimated from the classes' mean primitive
                                pairs) */
@@ -273,8 +274,9 @@ int dgf_fock_batch(dgf_batch *batch, const double *dmat_packed_device, double *f
 
 /* Per-class autotuner (no counterpart in Dalton): times every candidate
  * kernel of every quartet class of the plan for opt->thrs on the density
- * dmat_device (N x N, device) -- the cooperative team kernel and the
- * thread-per-quartet kernel in its A-chunk variants, FP64 and FP32 -- and
+ * dmat_device (N x N, device) -- the row kernel, the warp kernels, the
+ * cooperative team kernel and the thread-per-quartet kernel in its A-chunk
+ * variants, FP64 and FP32 -- and
  * keeps the fastest per class and precision in the context for later builds.
  * A JSON list of the timings is written to `report` (may be NULL). */
 int dgf_autotune(dgf_ctx *ctx, const double *dmat_device, const dgf_options *opt, void *stream, char *report,
@@ -286,8 +288,8 @@ int dgf_autotune(dgf_ctx *ctx, const double *dmat_device, const dgf_options *opt
 int dgf_copy_tuning(dgf_ctx *dst, const dgf_ctx *src);
 
 /* Pin the kernel of one quartet class (la lb|lc ld), as the autotuner would:
- * precision 64 or 32; variant -4 warp per quartet with FP64 tensor-core
- * (DMMA) transforms, -3 warp per quartet, -2 warp team, -1
+ * precision 64 or 32; variant -5 row kernel (FP64, single-primitive pairs),
+ * -4 warp per quartet with FP64 tensor-core (DMMA) transforms, -3 warp per quartet, -2 warp team, -1
  * cooperative team, 0.. thread-kernel chunk variants.  Launches the chosen
  * kernel cannot serve (e.g. a warp kernel restricted to one primitive pair
  * per side) fall back to the default kernel.  DGF_ERR_UNSUPPORTED when the
