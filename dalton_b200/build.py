@@ -79,7 +79,7 @@ def _generated_units():
     os.makedirs(gen, exist_ok=True)
     units = []
     for kind, header, macro, n, parts in (("jk", None, None, NUM_PAIR_CLASS, 5),
-                                          ("grad", "dgf_grad_kernel.cuh", "DGF_GRAD_CLASS", NUM_GRAD_CLASS, 0)):
+                                          ("grad", "dgf_grad_row.cuh", "DGF_GRAD_CLASS", NUM_GRAD_CLASS, 0)):
         for x in range(n):
             for y in range(x + 1):
                 for part in (range(parts) if parts else [None]):

@@ -459,7 +459,7 @@ constexpr int cls_lb(int X) { return X - cls_la(X) * (cls_la(X) + 1) / 2; }
 constexpr int kGradClasses = 6;  // pair classes up to (dd)
 
 typedef void (*GradLauncher)(const JKArgs &, int, int, cudaStream_t);
-extern GradLauncher g_grad_table[kGradClasses][kGradClasses];  // dgf_grad2e.cu; filled by DGF_GRAD_CLASS units
+extern GradLauncher g_grad_table[kGradClasses][kGradClasses];  // dgf_grad2e.cu; filled by DGF_GRAD_CLASS units (kets (ss), (ps))
 
 template <int LA, int LB, int LC, int LD>
 void launch_grad(const JKArgs &a, int grid, int block, cudaStream_t s) {
@@ -473,16 +473,3 @@ void launch_grad(const JKArgs &a, int grid, int block, cudaStream_t s) {
 
 }  // namespace grad
 }  // namespace dgf
-
-// Defines the static initialiser that fills entry (X, Y) of the gradient
-// table (one generated translation unit per class pair).
-#define DGF_GRAD_CLASS(X, Y)                                                                       \
-  namespace dgf {                                                                                  \
-  namespace grad {                                                                                 \
-  namespace {                                                                                      \
-  struct GradClassInit_##X##_##Y {                                                                 \
-    GradClassInit_##X##_##Y() { g_grad_table[X][Y] = &launch_grad<cls_la(X), cls_lb(X), cls_la(Y), cls_lb(Y)>; } \
-  } g_grad_class_init_##X##_##Y;                                                                   \
-  }                                                                                                \
-  }                                                                                                \
-  }
