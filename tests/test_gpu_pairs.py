@@ -1,0 +1,126 @@
+"""One-electron integrals and gradient on the working-basis pairs, the
+two-electron gradient's row and warp kernels, and the resolved form of
+contracted bases, against the oracle.
+
+Sizes and bases: s, p, d and f shells, spherical and Cartesian, general and
+segmented contractions, one molecule (tasks of one bra) and three."""
+import numpy as np
+import pytest
+
+from dalton_b200 import molecules
+from dalton_b200.basis import Molecule, build_basis
+from dalton_b200.fock import FockBuilder
+
+pytestmark = pytest.mark.gpu
+
+
+def _methane():
+    r = 0.63
+    return Molecule.from_angstrom(["C", "H", "H", "H", "H"],
+                                  [[0, 0, 0], [r, r, r], [-r, -r, r], [-r, r, -r], [r, -r, -r]])
+
+
+MOLS = {
+    "h2o_sto3g": (molecules.water_dalton_test, "STO-3G", True),
+    "h2o2_631gs": (lambda: molecules.water_cluster(2, seed=3), "6-31G*", True),
+    "h2o_631gs_cart": (molecules.water_dalton_test, "6-31G*", False),
+    "h2o3_dz": (lambda: molecules.water_cluster(3, seed=4), "cc-pVDZ", True),
+    "h2o_dz_cart": (molecules.water_dalton_test, "cc-pVDZ", False),
+    "h2o_aug": (molecules.water_dalton_test, "aug-cc-pVDZ", True),
+    "ch4_tz": (_methane, "cc-pVTZ", True),
+    "ch4_tz_cart": (_methane, "cc-pVTZ", False),
+}
+
+
+def _basis(name):
+    mol, basis, sph = MOLS[name]
+    return build_basis(mol(), basis, spherical=sph)
+
+
+def _density(n, seed, scale=0.1):
+    d = np.random.default_rng(seed).normal(size=(n, n)) * scale
+    return d + d.T
+
+
+@pytest.mark.parametrize("name", list(MOLS))
+def test_one_electron(cuda, orc, name):
+    bs = _basis(name)
+    fb = FockBuilder(bs)
+    for _ in range(2):  # the scratch is kept between calls
+        for x, y in zip(fb.oneint(), orc.oneint(bs)):
+            # rounding of contractions of up to ten primitives
+            assert np.abs(x - y).max() < 1e-13 * max(1.0, np.abs(y).max())
+        d, w = _density(bs.nbf, 1), _density(bs.nbf, 2)
+        g, ref = fb.grad1e(d, w), orc.grad1e(bs, d, w)
+        assert np.abs(g - ref).max() < 1e-14 * bs.nbf * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("name", [n for n in MOLS if not n.startswith("ch4")])
+@pytest.mark.parametrize("hfx", [1.0, 0.0, 0.3])
+def test_bilinear_gradient(cuda, orc, name, hfx):
+    """K(D1, D2) = [K(D1 + D2, D1 + D2) - K(D1 - D2, D1 - D2)] / 4 with the
+    oracle's quadratic form; D1 = D2 through the same entry point."""
+    import torch
+
+    from dalton_b200.grad import grad2e_bilinear
+
+    bs = _basis(name)
+    fb = FockBuilder(bs)
+    d1, d2 = _density(bs.nbf, 5, 0.05), _density(bs.nbf, 6, 0.05)
+    dev = lambda m: torch.tensor(m, device=cuda)
+    ref = (orc.grad2e(bs, d1 + d2, hfx, 1e-12) - orc.grad2e(bs, d1 - d2, hfx, 1e-12)) / 4
+    # Schwarz-screened quartets differ (working basis, primitives): 1e-10 as
+    # the gradient's parity elsewhere
+    for _ in range(2):
+        assert np.abs(grad2e_bilinear(fb, dev(d1), dev(d2), hfx).cpu().numpy() - ref).max() < 1e-10
+    same = grad2e_bilinear(fb, dev(d1), dev(d1), hfx).cpu().numpy()
+    assert np.abs(same - orc.grad2e(bs, d1, hfx, 1e-12)).max() < 1e-10
+
+
+@pytest.mark.parametrize("name", ["h2o_sto3g", "h2o2_631gs", "h2o_631gs_cart"])
+def test_resolved_contractions(cuda, orc, name):
+    """Direct builds and gradients of segmented bases run in the resolved
+    form until a kernel is pinned on the context; both against the oracle's
+    unscreened build, the resolved one to the accuracy of its tighter
+    threshold."""
+    import torch
+
+    bs = _basis(name)
+    res, con = FockBuilder(bs), FockBuilder(bs)
+    con.set_class_kernel((1, 0, 0, 0), 0)  # what it would choose anyway: now serves all calls itself
+    d = _density(bs.nbf, 8)
+    ref = orc.fock(bs, d, 13, 1.0, 0.0)
+    f, g = res.herfck(d, 13), con.herfck(d, 13)
+    assert res.last_stats["prim_quartets"] == res.last_stats["quartets_total"]
+    assert con.last_stats["prim_quartets"] > con.last_stats["quartets_total"]
+    assert np.abs(g - ref).max() < 1e-10
+    assert np.abs(f - ref).max() < 1e-12 * max(1.0, np.abs(ref).max())
+    assert np.abs(res.herfck(d, 13, ifthrs=10) - con.herfck(d, 13, ifthrs=10)).max() < 1e-7
+    assert np.abs(res.grad2e(d) - con.grad2e(d)).max() < 1e-10
+    # a store keeps contracted blocks; stored and direct builds agree
+    n = res.store_integrals()
+    assert n == con.store_integrals()
+    dt = torch.tensor(d, device=cuda)
+    assert float((res.herfck_stored(dt) - res.herfck_device(dt)).abs().max()) < 1e-11
+
+
+@pytest.mark.parametrize("basis", ["6-31G*", "cc-pVDZ"])
+def test_batch_rows(cuda, basis):
+    """Batched builds with the row kernels: molecules of one to five waters,
+    FP64 and mixed, replayed with new densities."""
+    import torch
+
+    from dalton_b200.batch import BatchBuilder
+
+    fbs = [FockBuilder(build_basis(molecules.water_cluster(n, seed=n), basis)) for n in (1, 5, 2, 1, 3)]
+    bb = BatchBuilder(fbs)
+    out = None
+    for seed in (1, 2):
+        ds = [torch.tensor(_density(fb.nbf, 10 * seed + k), device=cuda) for k, fb in enumerate(fbs)]
+        ref = [fb.herfck_device(d) for fb, d in zip(fbs, ds)]
+        for graph in (False, True, True):
+            fp = bb.herfck_batch(bb.pack(ds), out, use_graph=graph)
+            for a, b in zip(bb.unpack(fp), ref):
+                assert float((a - b).abs().max()) < 1e-14 * a.shape[0] * max(1.0, float(b.abs().max()))
+        fm = bb.unpack(bb.herfck_batch(bb.pack(ds), use_graph=False, mixed_cutoff=1e-7))
+        assert max(float((a - b).abs().max()) for a, b in zip(fm, ref)) < 1e-6
