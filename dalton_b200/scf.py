@@ -116,15 +116,16 @@ def rhf(bs: BasisSet, fb: FockBuilder | None = None, conv: float = 1e-8, maxiter
         n = len(errs)
         Fx = F
         if n >= 2:
+            # all inner products and the extrapolation as two products of the
+            # stacked matrices: one launch each, not one per pair of errors
             Bm = -torch.ones((n + 1, n + 1), dtype=F.dtype, device=dev)
             Bm[n, n] = 0.0
-            for i in range(n):
-                for j in range(n):
-                    Bm[i, j] = torch.sum(errs[i] * errs[j])
+            E = torch.stack(errs).reshape(n, -1)
+            Bm[:n, :n] = E @ E.T
             rhs = torch.zeros(n + 1, dtype=F.dtype, device=dev)
             rhs[n] = -1.0
             cvec = torch.linalg.solve(Bm, rhs)[:n]
-            Fx = sum(c * f for c, f in zip(cvec, focks))
+            Fx = torch.tensordot(cvec, torch.stack(focks), dims=1)
         eps, C = solve(Fx)
         D = 2.0 * C[:, :nocc] @ C[:, :nocc].T
     eps, C = solve(F)
