@@ -21,6 +21,7 @@
 
 #include "dgf_ctx.h"
 #include "dgf_md.cuh"
+#include "dgf_pack.h"
 
 using namespace dgf;
 
@@ -579,7 +580,7 @@ static int batch_enqueue(dgf_batch *b, const double *din, double *fout, double h
     const bool row = bp.row_ntask > 0 && row_slot < kRowSlots && (choice == kDefaultVariant || choice == kRowVariant) &&
                      !(mixed && b->split_ok[bp.X][bp.Y] == 2);
     if (row) {
-      const ClassKernel &k = jk_row_entry(bp.X, bp.Y);
+      const ClassKernel &k = g_row_batch[bp.X][bp.Y];
       a.mode = 0;
       a.counters = b->d_cnt + 4 * (slot++ % kCounterSlots);
       a.boys_fine = b->d_fine + (size_t)Lq * kFineDoubles;

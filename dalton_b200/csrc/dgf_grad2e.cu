@@ -207,15 +207,17 @@ static int grad_impl(dgf_ctx *c, const double *d1, const double *d2, double hfx,
       cudaEventRecord(e0, ls);
     }
     const GradEntry &g = g_grad_entry[cp.X][cp.Y];
-    if (!g.row) {
-      g.launch(a, pg, (int)std::max<int64_t>(1, std::min<int64_t>((cp.nquartet + g.wpb - 1) / g.wpb, c->nsm * 16)), ls);
-    } else if (cp.row_ntask > 0 && nrow < kRowSlots) {
+    if (g.row && cp.row_ntask > 0 && nrow < kRowSlots) {
       a.row_bra = c->d_row_bra + c->cls_off[cp.X];
       a.row_tasks = c->d_row_tasks + cp.row_off;
       a.row_task0 = 0;
       a.row_task1 = cp.row_ntask;
       a.row_work = work + nrow++;
-      g.launch(a, pg, std::max(1, std::min((cp.row_ntask + g.wpb - 1) / g.wpb, c->nsm * g.blocks)), ls);
+      g.row(a, pg, std::max(1, std::min((cp.row_ntask + g.row_warps - 1) / g.row_warps, c->nsm * g.row_blocks)), ls);
+    } else if (g.warp) {
+      g.warp(a, pg,
+             (int)std::max<int64_t>(1, std::min<int64_t>((cp.nquartet + g.warp_warps - 1) / g.warp_warps, c->nsm * 16)),
+             ls);
     } else {  // contracted pairs: one thread per quartet, straight into the gradient
       g_grad_table[cp.X][cp.Y](
           a, (int)std::max<int64_t>(1, std::min<int64_t>((cp.nquartet + kGradBlock - 1) / kGradBlock, c->nsm * 8)),

@@ -17,10 +17,10 @@
 // (A then B), which grad_pairs_kernel sums over the atoms: neighbouring lanes
 // add to different addresses, where the molecule's few atoms would be hot.
 //
-// grad_row_kernel: kets (ss) and (ps), single-primitive pairs; the row
-// kernels' tiles (dgf_jk_row.cuh): a warp on the bras of one A shell, one ket
-// per lane.  grad_warp_kernel: the other kets; one warp per quartet, a lane
-// on each ket component, R_tuv in shared memory.
+// grad_row_kernel: small kets, single-primitive pairs; the row kernels' tiles
+// (dgf_jk_row.cuh): a warp on the bras of one A shell, one ket per lane.
+// grad_warp_kernel: the other kets; one warp per quartet, a lane on each ket
+// component, R_tuv in shared memory.
 #pragma once
 
 #include "dgf_grad_kernel.cuh"
@@ -73,7 +73,6 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : (LA + LB +
   constexpr int L = LA + LB + LC + LD, LAB = LA + LB, LCD = LC + LD;
   constexpr int NA = S::NA, NB = S::NB, NC = ncart(LC), ND = ncart(LD), NCD = NC * ND;
   constexpr int EA = (LA + 1) * (LB + 1) * (LAB + 1), EC = (LC + 1) * (LD + 1) * (LCD + 1);
-  static_assert(LD == 0 && LC <= 1, "kets (ss) and (ps)");
   constexpr unsigned full = 0xffffffffu;
   extern __shared__ double sm[];
   for (int i = threadIdx.x; i < kBoysTableDoubles; i += blockDim.x) sm[i] = a.boys[i];
@@ -210,21 +209,24 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : (LA + LB +
 #pragma unroll
         for (int k = 0; k < 3; ++k) herm_e<LA, LB, 1, double>(0.5 / p, w[S::kPA + k], w[S::kPB + k], e1[k]);
         double gP[3] = {0.0, 0.0, 0.0}, gX[3] = {0.0, 0.0, 0.0}, e0 = 0.0;
-        static_for<NC>([&](auto C_) {
-          constexpr int c = decltype(C_)::value;  // D is s: the component pair is c
-          constexpr int c0 = cart_x(LC, c), c1 = cart_y(LC, c), c2 = cart_z(LC, c);
+        static_for<NCD>([&](auto CD_) {
+          constexpr int c = decltype(CD_)::value / ND, d = decltype(CD_)::value % ND;
+          constexpr int k0 = cart_e(LC, c, 0), k1 = cart_e(LC, c, 1), k2 = cart_e(LC, c, 2);
+          constexpr int l0 = cart_e(LD, d, 0), l1 = cart_e(LD, d, 1), l2 = cart_e(LD, d, 2);
+          auto K = [&](int k, int tt) {
+            return e2[k][(cart_e(LC, c, k) * (LD + 1) + cart_e(LD, d, k)) * (LCD + 1) + tt];
+          };
           // ket transform, one index past the bra's range
           double xk[n3(LAB + 1)];
 #pragma unroll
           for (int e = 0; e < n3(LAB + 1); ++e) xk[e] = 0.0;
 #pragma unroll
-          for (int ta = 0; ta <= c0; ++ta)
+          for (int ta = 0; ta <= k0 + l0; ++ta)
 #pragma unroll
-            for (int na = 0; na <= c1; ++na)
+            for (int na = 0; na <= k1 + l1; ++na)
 #pragma unroll
-              for (int fa2 = 0; fa2 <= c2; ++fa2) {
-                const double e3 = e2[0][c0 * (LCD + 1) + ta] * e2[1][c1 * (LCD + 1) + na] *
-                                  e2[2][c2 * (LCD + 1) + fa2];
+              for (int fa2 = 0; fa2 <= k2 + l2; ++fa2) {
+                const double e3 = K(0, ta) * K(1, na) * K(2, fa2);
 #pragma unroll
                 for (int tt = 0; tt <= LAB + 1; ++tt)
 #pragma unroll
@@ -240,9 +242,9 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : (LA + LB +
           for (int e = 0; e < n3(LAB); ++e) W[e] = 0.0;
           static_for<NA * NB>([&](auto AB_) {
             constexpr int ab = decltype(AB_)::value, ia = ab / NB, jb = ab % NB;
-            const double g = 2.0 * (w[S::kAB + ab] * cd2[c] + w[S::kAB + NA * NB + ab] * cd1[c]) -
-                             h * (ac1[ia * NC + c] * bd2[jb] + ac2[ia * NC + c] * bd1[jb] +
-                                  ad1[ia] * bc2[jb * NC + c] + ad2[ia] * bc1[jb * NC + c]);
+            const double g = 2.0 * (w[S::kAB + ab] * cd2[c * ND + d] + w[S::kAB + NA * NB + ab] * cd1[c * ND + d]) -
+                             h * (ac1[ia * NC + c] * bd2[jb * ND + d] + ac2[ia * NC + c] * bd1[jb * ND + d] +
+                                  ad1[ia * ND + d] * bc2[jb * NC + c] + ad2[ia * ND + d] * bc1[jb * NC + c]);
             auto E = [&](int k, int tt) {
               return e1[k][(cart_e(LA, ia, k) * (LB + 1) + cart_e(LB, jb, k)) * (LAB + 1) + tt];
             };
@@ -291,13 +293,32 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : (LA + LB +
                 gP[2] += we * xk[tuv_index(tt, u, v + 1)];
               }
           e0 += s;
-          // a p function of C lowers to -(d/q) (00|: its dE/dY
-          if constexpr (LC == 1) {
-            double y = 0.0;
+          // lowered ket coefficients: dE/dY
+          static_for<3>([&](auto K_) {
+            constexpr int k = decltype(K_)::value, ck = cart_e(LC, c, k), dk = cart_e(LD, d, k);
+            if constexpr (ck + dk > 0) {
+              constexpr int m0 = k0 + l0 - (k == 0), m1 = k1 + l1 - (k == 1), m2 = k2 + l2 - (k == 2);
 #pragma unroll
-            for (int e = 0; e < n3(LAB); ++e) y += W[e] * R[e];
-            gY[c] += (f2c - 1.0) * y;  // -d/q
-          }
+              for (int ta = 0; ta <= m0; ++ta)
+#pragma unroll
+                for (int na = 0; na <= m1; ++na)
+#pragma unroll
+                  for (int fa2 = 0; fa2 <= m2; ++fa2) {
+                    const double x0 = k == 0 ? lowered<LC, LD>(e2[0], ck, dk, ta, f2c - 1.0, f2c) : K(0, ta);
+                    const double x1 = k == 1 ? lowered<LC, LD>(e2[1], ck, dk, na, f2c - 1.0, f2c) : K(1, na);
+                    const double x2 = k == 2 ? lowered<LC, LD>(e2[2], ck, dk, fa2, f2c - 1.0, f2c) : K(2, fa2);
+                    double y = 0.0;
+#pragma unroll
+                    for (int tt = 0; tt <= LAB; ++tt)
+#pragma unroll
+                      for (int u = 0; u <= LAB - tt; ++u)
+#pragma unroll
+                        for (int v = 0; v <= LAB - tt - u; ++v)
+                          y += W[tuv_index(tt, u, v)] * R[tuv_index(tt + ta, u + na, v + fa2)];
+                    gY[k] += x0 * x1 * x2 * y;
+                  }
+            }
+          });
         });
         // X = A - B = (P - B) - (P - A)
         double fB[3];
@@ -663,76 +684,82 @@ __global__ void __launch_bounds__(128) grad_warp_kernel(const __grid_constant__ 
   }
 }
 
-// Kernels of a class pair: the row kernel for kets (ss) and (ps) (needs the
-// plan entry's row tasks), the warp kernel for the others.
+// Kernels of a class pair (null: none): the row kernel takes plan entries
+// with row tasks; the warp kernel any; the thread kernel (dgf_grad_kernel.cuh)
+// the contracted pairs of classes without a warp kernel.
+typedef void (*PairGradLauncher)(const JKArgs &, const PairGrad &, int grid, cudaStream_t);
 struct GradEntry {
-  void (*launch)(const JKArgs &, const PairGrad &, int grid, cudaStream_t);
-  bool row;
-  int wpb;          // warps per block
-  int blocks;       // row: resident blocks per SM
+  PairGradLauncher row, warp;
+  int row_warps, row_blocks;  // warps per block, resident blocks per SM
+  int warp_warps;
   cudaError_t (*prepare)();
 };
 extern GradEntry g_grad_entry[kGradClasses][kGradClasses];  // dgf_grad2e.cu; filled by DGF_GRAD_CLASS units
 
-template <int LA, int LB, int LC, int LD, bool SPH>
-void *grad_kernel_ptr() {
-  if constexpr (ncart(LC) * ncart(LD) <= 3)
-    return (void *)grad_row_kernel<LA, LB, LC, LD, SPH>;
+// Classes with the row kernel: kets (ss) and (ps), where the warp kernel
+// would leave most lanes without a ket component, and (pp) and (ds) kets up to
+// L = 4 (above, a thread's R_tuv and tables spill more than they save, and
+// the unrolled code takes minutes to compile).   On (H2O)9 / cc-pVDZ, warp then
+// row kernel: (ds|pp) 2.88 and 0.15 ms, (pp|pp) 1.45 and 0.17, (ds|ds) 1.00 and
+// 0.08.
+constexpr bool grad_by_row(int LA, int LB, int LC, int LD) {
+  return ncart(LC) * ncart(LD) <= 3 || LA + LB + LC + LD <= 4;
+}
+// Classes with the warp kernel: the other kets; it also serves the contracted
+// pairs of the row kernel's classes with more than three ket components.
+constexpr bool grad_by_warp(int LC, int LD) { return ncart(LC) * ncart(LD) > 3; }
+
+template <int LA, int LB, int LC, int LD>
+void launch_grad_row(const JKArgs &a, const PairGrad &pg, int grid, cudaStream_t s) {
+  using R = RowGrad<LA, LB>;
+  if (a.spherical)
+    grad_row_kernel<LA, LB, LC, LD, true><<<grid, R::kBlock, R::smem(), s>>>(a, pg);
   else
-    return (void *)grad_warp_kernel<LA, LB, LC, LD, SPH>;
+    grad_row_kernel<LA, LB, LC, LD, false><<<grid, R::kBlock, R::smem(), s>>>(a, pg);
 }
 
 template <int LA, int LB, int LC, int LD>
-constexpr size_t grad_smem() {
-  if constexpr (ncart(LC) * ncart(LD) <= 3)
-    return RowGrad<LA, LB>::smem();
+void launch_grad_warp(const JKArgs &a, const PairGrad &pg, int grid, cudaStream_t s) {
+  using W = WarpGrad<LA, LB, LC, LD>;
+  if (a.spherical)
+    grad_warp_kernel<LA, LB, LC, LD, true><<<grid, 32 * W::WPB, W::smem(W::WPB), s>>>(a, pg);
   else
-    return WarpGrad<LA, LB, LC, LD>::smem(WarpGrad<LA, LB, LC, LD>::WPB);
-}
-
-template <int LA, int LB, int LC, int LD>
-void launch_grad_entry(const JKArgs &a, const PairGrad &pg, int grid, cudaStream_t s) {
-  constexpr size_t smem = grad_smem<LA, LB, LC, LD>();
-  if constexpr (ncart(LC) * ncart(LD) <= 3) {
-    if (a.spherical)
-      grad_row_kernel<LA, LB, LC, LD, true><<<grid, RowGrad<LA, LB>::kBlock, smem, s>>>(a, pg);
-    else
-      grad_row_kernel<LA, LB, LC, LD, false><<<grid, RowGrad<LA, LB>::kBlock, smem, s>>>(a, pg);
-  } else {
-    using W = WarpGrad<LA, LB, LC, LD>;
-    if (a.spherical)
-      grad_warp_kernel<LA, LB, LC, LD, true><<<grid, 32 * W::WPB, smem, s>>>(a, pg);
-    else
-      grad_warp_kernel<LA, LB, LC, LD, false><<<grid, 32 * W::WPB, smem, s>>>(a, pg);
-  }
+    grad_warp_kernel<LA, LB, LC, LD, false><<<grid, 32 * W::WPB, W::smem(W::WPB), s>>>(a, pg);
 }
 
 template <int LA, int LB, int LC, int LD>
 cudaError_t prepare_grad() {
-  constexpr int smem = (int)grad_smem<LA, LB, LC, LD>();
-  cudaError_t e = cudaFuncSetAttribute(grad_kernel_ptr<LA, LB, LC, LD, true>(),
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(grad_kernel_ptr<LA, LB, LC, LD, false>(), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cudaSuccess;
+  auto allow = [&](auto *f, size_t smem) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  };
+  if constexpr (grad_by_row(LA, LB, LC, LD)) {
+    allow(grad_row_kernel<LA, LB, LC, LD, true>, RowGrad<LA, LB>::smem());
+    allow(grad_row_kernel<LA, LB, LC, LD, false>, RowGrad<LA, LB>::smem());
+  }
+  if constexpr (grad_by_warp(LC, LD)) {
+    using W = WarpGrad<LA, LB, LC, LD>;
+    allow(grad_warp_kernel<LA, LB, LC, LD, true>, W::smem(W::WPB));
+    allow(grad_warp_kernel<LA, LB, LC, LD, false>, W::smem(W::WPB));
+  }
   return e;
 }
 
 template <int X, int Y>
 void fill_grad() {
   constexpr int LA = cls_la(X), LB = cls_lb(X), LC = cls_la(Y), LD = cls_lb(Y);
-  constexpr bool row = ncart(LC) * ncart(LD) <= 3;
   GradEntry &e = g_grad_entry[X][Y];
-  e.launch = &launch_grad_entry<LA, LB, LC, LD>;
   e.prepare = &prepare_grad<LA, LB, LC, LD>;
-  e.row = row;
-  if constexpr (row) {
-    e.wpb = RowGrad<LA, LB>::kWarps;
-    e.blocks = LA + LB + LC + LD <= 1 ? 4 : LA + LB + LC + LD <= 2 ? 3 : 2;
-    // contracted bras of these classes: one thread per quartet (dgf_grad_kernel.cuh)
-    g_grad_table[X][Y] = &launch_grad<LA, LB, LC, LD>;
+  if constexpr (grad_by_row(LA, LB, LC, LD)) {
+    e.row = &launch_grad_row<LA, LB, LC, LD>;
+    e.row_warps = RowGrad<LA, LB>::kWarps;
+    e.row_blocks = LA + LB + LC + LD <= 1 ? 4 : LA + LB + LC + LD <= 2 ? 3 : 2;
+  }
+  if constexpr (grad_by_warp(LC, LD)) {
+    e.warp = &launch_grad_warp<LA, LB, LC, LD>;
+    e.warp_warps = WarpGrad<LA, LB, LC, LD>::WPB;
   } else {
-    e.wpb = WarpGrad<LA, LB, LC, LD>::WPB;
-    e.blocks = 0;
+    g_grad_table[X][Y] = &launch_grad<LA, LB, LC, LD>;
   }
 }
 

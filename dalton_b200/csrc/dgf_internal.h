@@ -169,15 +169,16 @@ struct JKArgs {
   const double *ks_pp;
   int64_t ks_stride;
   int ks_base;
-  // row kernels (dgf_jk_row.cuh): the fine Boys table of order L, the bra
-  // pairs in row order (class-relative positions), the tasks {first bra,
-  // bras, first 32-ket chunk, chunks} of this launch, the kets of the plan
-  // entry, and the task counters (one per A chunk, zero at the launch)
+  // row and pack kernels (dgf_jk_row.cuh, dgf_jk_pack.cuh): the fine Boys
+  // table of order L, the bra pairs in row order (class positions), the tasks
+  // {first bra, bras | 32-ket chunks << 16, first ket, end of the kets} and
+  // this launch's range of them, and the task counters (one per A chunk, zero
+  // at the launch)
   const double *boys_fine;
   const int *row_bra;
   const int4 *row_tasks;
   unsigned *row_work;
-  int row_task0, row_task1, row_nket;
+  int row_task0, row_task1;
   // gradient mode (dgf_grad2e): densities D1, D2 (N*N) and grad (natom*3)
   const double *G1, *G2;
   double *grad;

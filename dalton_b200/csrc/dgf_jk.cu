@@ -13,6 +13,7 @@ JKEntry g_jk_table[kNumPairClass][kNumPairClass];
 PackEntry g_pack_table[kNumPairClass][kNumPairClass];
 FragEntry g_frag_table[kNumPairClass];
 ClassKernel g_row_stored[kNumPairClass][kNumPairClass];
+ClassKernel g_row_batch[kNumPairClass][kNumPairClass];
 
 namespace {
 const ClassKernel kNone{nullptr, 0, 0, 0, 0, 0};

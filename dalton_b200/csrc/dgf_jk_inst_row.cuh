@@ -23,9 +23,9 @@ constexpr int row_chunks(int LA, int LB, int LC, int LD) {
 
 constexpr int kRowCarveoutPercent = 60;
 
-template <int LA, int LB, int LC, int LD, int CA>
+template <int LA, int LB, int LC, int LD, int CA, bool BT>
 void launch_row(const JKArgs &a, int grid, int block, size_t smem, cudaStream_t s) {
-  jk_row_kernel<LA, LB, LC, LD, CA><<<dim3(grid, CA), block, smem, s>>>(a);
+  jk_row_kernel<LA, LB, LC, LD, CA, BT><<<dim3(grid, CA), block, smem, s>>>(a);
 }
 
 template <int LA, int LB, int LC, int LD, int CA>
@@ -43,15 +43,18 @@ cudaError_t prepare_row() {
   if constexpr (CA > 0) {
     using S = row::Shape<LA, LB, LC, LD, CA>;
     static_assert(S::kR == row_max_bras(X) && CA <= kRowChunksMax && S::L <= kFineMaxM, "row kernel limits");
-    cudaError_t e = cudaFuncSetAttribute(jk_row_kernel<LA, LB, LC, LD, CA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)S::smem());
     // One carveout for all of them (it fits their resident blocks, and the
     // rest stays L1 cache for the density gathers): an SM that changes it
     // between two kernels drains first.
     static_assert((S::smem() + 1024) * S::kMinBlocks <= (size_t)kRowCarveoutPercent * 228 * 1024 / 100, "row carveout");
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(jk_row_kernel<LA, LB, LC, LD, CA>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               kRowCarveoutPercent);
+    cudaError_t e = cudaSuccess;
+    auto prepare = [&](auto *f) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem());
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, kRowCarveoutPercent);
+    };
+    prepare(jk_row_kernel<LA, LB, LC, LD, CA, false>);
+    prepare(jk_row_kernel<LA, LB, LC, LD, CA, true>);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(jk_row_stored_kernel<LA, LB, LC, LD, CA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)row_stored_smem<LA, LB, LC, LD, CA>());
@@ -67,7 +70,8 @@ void fill_row() {
   e.prepare[3] = &prepare_row<X, Y>;
   if constexpr (CA > 0) {
     using S = row::Shape<LA, LB, LC, LD, CA>;
-    e.row = ClassKernel{&launch_row<LA, LB, LC, LD, CA>, S::kBlock, S::smem(), CA, S::kMinBlocks, kKindRow};
+    e.row = ClassKernel{&launch_row<LA, LB, LC, LD, CA, false>, S::kBlock, S::smem(), CA, S::kMinBlocks, kKindRow};
+    g_row_batch[X][Y] = ClassKernel{&launch_row<LA, LB, LC, LD, CA, true>, S::kBlock, S::smem(), CA, S::kMinBlocks, kKindRow};
     g_row_stored[X][Y] = ClassKernel{&launch_row_stored<LA, LB, LC, LD, CA>, kRowStoredBlock,
                                      row_stored_smem<LA, LB, LC, LD, CA>(), CA, 2, kKindRow};
   }

@@ -168,8 +168,13 @@ struct Shape {
   static constexpr size_t smem() { return ((size_t)kFineDoubles + (size_t)kWarps * kPerWarp) * 8; }
 };
 
-// ST: digestion of stored integrals (JKArgs::store_in) instead of evaluation.
-template <int LA, int LB, int LC, int LD, int CA, int CH, bool ST>
+// What a row kernel runs on: the quartets of one molecule, those of a batch
+// (each segment has its own matrices: their size and place take registers,
+// 15% of the time of the s kernels, so that the form is its own), or the
+// stored integrals of one molecule.
+enum { kEval = 0, kBatch = 1, kStored = 2 };
+
+template <int LA, int LB, int LC, int LD, int CA, int CH, int FORM>
 __device__ __forceinline__ void row_body(const JKArgs &a, const double *tab, double *wsm, unsigned long long &cnt_q,
                                          unsigned long long &cnt_s) {
   using S = Shape<LA, LB, LC, LD, CA>;
@@ -178,17 +183,23 @@ __device__ __forceinline__ void row_body(const JKArgs &a, const double *tab, dou
   constexpr int FA = chunk_size(LA, CA, CH), FB = S::FB, FC = S::FC, FD = S::FD;
   constexpr int EA = (LA + 1) * (LB + 1) * (LAB + 1), EC = (LC + 1) * (LD + 1) * (LCD + 1);
   constexpr unsigned full = 0xffffffffu;
+  constexpr bool ST = FORM == kStored, BT = FORM == kBatch;
   const int lane = threadIdx.x & 31;
   double *jab = wsm + S::kR * S::kRow;
   const int jslot = warp_slot<FA * FB>(lane);
   auto afun = [](int x) { return chunk_fun(LA, CA, CH, x); };  // function of A of the chunk's row x
   const double js = a.jscale[0], ks = -a.kscale[0];
   int seg = -1, aoA = 0, nb = 0, blkA = 0;
-  int N = 0;  // the segment's molecule: its matrices' size and place
-  const double *Dm = a.D, *Dsm = a.Ds;
-  double *Fm = a.Fh;
+  int Nb = 0;  // batches: size and place of the segment's matrices
+  int64_t db = 0;
+#define DGF_ROW_MATRICES                                  \
+  const int N = BT ? Nb : a.nbf;                          \
+  const double *Dm = BT ? a.D + db : a.D, *Dsm = BT ? a.Ds + db : a.Ds; \
+  double *Fm = BT ? a.Fh + db : a.Fh;                     \
+  (void)Dm, (void)Dsm, (void)Fm
   // J_ab of the staged bras to the half Fock matrix
   auto flush_jab = [&]() {
+    DGF_ROW_MATRICES;
     __syncwarp();
     if (js != 0.0)
       for (int e = lane; e < nb * FA * FB; e += 32) {
@@ -209,13 +220,12 @@ __device__ __forceinline__ void row_body(const JKArgs &a, const double *tab, dou
       if (seg >= 0) flush_jab();
       seg = tk.x;
       nb = tk.y & 0xffff;
-      {
+      if (BT) {
         const PairRec b0 = load_pair_fock(a.bra + __ldg(a.row_bra + seg));
-        N = b0.nbfm;
-        Dm = a.D + b0.dbase;
-        Dsm = a.Ds + b0.dbase;
-        Fm = a.Fh + b0.dbase;
+        Nb = b0.nbfm;
+        db = b0.dbase;
       }
+      DGF_ROW_MATRICES;
       if (lane < nb) {
         const int ib = __ldg(a.row_bra + seg + lane);
         const PairRec br = load_pair_fock(a.bra + ib);
@@ -265,6 +275,7 @@ __device__ __forceinline__ void row_body(const JKArgs &a, const double *tab, dou
       blkA = __shfl_sync(full, blkA, 0);
       __syncwarp();
     }
+    DGF_ROW_MATRICES;
     const int kend = min(tk.w, tk.z + 32 * (tk.y >> 16));
     for (int ic0 = tk.z; ic0 < kend; ic0 += 32) {
       const int ic = ic0 + lane;
@@ -572,14 +583,16 @@ __device__ __forceinline__ void row_body(const JKArgs &a, const double *tab, dou
   if (seg >= 0) flush_jab();
 }
 
-template <int LA, int LB, int LC, int LD, int CA, int CH, bool ST>
+#undef DGF_ROW_MATRICES
+
+template <int LA, int LB, int LC, int LD, int CA, int CH, int FORM>
 __device__ __forceinline__ void row_dispatch(int chunk, const JKArgs &a, const double *tab, double *wsm,
                                              unsigned long long &q, unsigned long long &s) {
   if constexpr (CH < CA) {
     if (chunk == CH)
-      row_body<LA, LB, LC, LD, CA, CH, ST>(a, tab, wsm, q, s);
+      row_body<LA, LB, LC, LD, CA, CH, FORM>(a, tab, wsm, q, s);
     else
-      row_dispatch<LA, LB, LC, LD, CA, CH + 1, ST>(chunk, a, tab, wsm, q, s);
+      row_dispatch<LA, LB, LC, LD, CA, CH + 1, FORM>(chunk, a, tab, wsm, q, s);
   }
 }
 
@@ -604,7 +617,7 @@ __device__ __forceinline__ void add_counts(const JKArgs &a, unsigned long long n
 
 // CA > 1: blockIdx.y takes one of CA chunks of A's functions, which bounds the
 // registers; each chunk forms R_tuv and the ket transform again.
-template <int LA, int LB, int LC, int LD, int CA>
+template <int LA, int LB, int LC, int LD, int CA, bool BT>
 __global__ void __launch_bounds__(row::Shape<LA, LB, LC, LD, CA>::kBlock, row::Shape<LA, LB, LC, LD, CA>::kMinBlocks)
     jk_row_kernel(const __grid_constant__ JKArgs a) {
   using S = row::Shape<LA, LB, LC, LD, CA>;
@@ -612,7 +625,7 @@ __global__ void __launch_bounds__(row::Shape<LA, LB, LC, LD, CA>::kBlock, row::S
   for (int i = threadIdx.x; i < kFineDoubles; i += blockDim.x) sm[i] = a.boys_fine[i];
   __syncthreads();
   unsigned long long cnt_q = 0, cnt_s = 0;
-  row::row_dispatch<LA, LB, LC, LD, CA, 0, false>(blockIdx.y, a, sm,
+  row::row_dispatch<LA, LB, LC, LD, CA, 0, BT ? row::kBatch : row::kEval>(blockIdx.y, a, sm,
                                            sm + kFineDoubles + (size_t)(threadIdx.x >> 5) * S::kPerWarp, cnt_q, cnt_s);
   row::add_counts(a, cnt_q, cnt_q, cnt_s);  // one primitive quartet each
 }
@@ -626,7 +639,7 @@ __global__ void __launch_bounds__(kRowStoredBlock, 2) jk_row_stored_kernel(const
   using S = row::Shape<LA, LB, LC, LD, CA>;
   extern __shared__ double sm[];
   unsigned long long cnt_q = 0, cnt_s = 0;
-  row::row_dispatch<LA, LB, LC, LD, CA, 0, true>(blockIdx.y, a, nullptr, sm + (size_t)(threadIdx.x >> 5) * S::kPerWarp,
+  row::row_dispatch<LA, LB, LC, LD, CA, 0, row::kStored>(blockIdx.y, a, nullptr, sm + (size_t)(threadIdx.x >> 5) * S::kPerWarp,
                                                  cnt_q, cnt_s);
   row::add_counts(a, cnt_q, 0, cnt_s);
 }

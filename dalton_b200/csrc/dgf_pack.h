@@ -27,6 +27,7 @@ struct FragEntry {
 extern FragEntry g_frag_table[kNumPairClass];
 
 extern ClassKernel g_row_stored[kNumPairClass][kNumPairClass];  // launch null: none
+extern ClassKernel g_row_batch[kNumPairClass][kNumPairClass];   // the batches' form
 
 constexpr int kPackVariant = -6;
 constexpr int kKindPack = 10;  // ClassKernel::kind
