@@ -24,7 +24,7 @@
 // Boys function: F_L from a table of degree-7 polynomials on intervals of
 // 1/8 (Chebyshev interpolants), e^-T by its Taylor series about the
 // interval's midpoint from the same table row; above T = 40 the asymptotic
-// F_0 and upward recursion.
+// F_0 and upward recursion (boys_scaled).
 #pragma once
 
 #include "dgf_select.cuh"
@@ -32,11 +32,23 @@
 namespace dgf {
 namespace row {
 
-// F_L and e^-T, ..., F_0 on T < kBoysTmax from the fine table, rows of
-// kFineStride doubles: 8 coefficients in x in [-1, 1], e^-mid, unused.
+// The scaled R^n_000 = K (-2 alpha)^n F_n(alpha r2) / sqrt(B), n = 0 .. M, for
+// alpha = A / B (plain operator: A = p q, B = p + q; the attenuated one has
+// A = p q mu^2, B = (p + q) mu^2 + p q, K times mu).  One reciprocal square
+// root serves both ranges: of B below T = alpha r2 = 40, of A r2 above it,
+// where R^0 = K sqrt(pi / (A r2)) / 2 and each higher order divides by r2;
+// the lanes of a warp usually fall on both sides.
+// Below, F_M comes from the fine table (rows of kFineStride doubles: 8
+// coefficients in x in [-1, 1], e^-mid, unused).
 template <int M>
-__device__ __forceinline__ void boys_fine(double T, const double *__restrict__ tab, double *F) {
-  if (T < kBoysTmax) {
+__device__ __forceinline__ void boys_scaled(double A, double B, double r2, double K, const double *__restrict__ tab,
+                                            double *F) {
+  const double ar = A * r2;
+  const bool large = ar >= kBoysTmax * B;
+  const double y = rsqrt(large ? ar : B), y2 = y * y;
+  double s = K * y;
+  if (!large) {
+    const double alpha = A * y2, T = fmin(alpha * r2, kBoysTmax * (1.0 - 1e-15));
     const int i = (int)(T * kFinePerUnit);
     const double u = T - ((double)i + 0.5) * (1.0 / kFinePerUnit);  // |u| <= 1/16
     const double x = u * (2.0 * kFinePerUnit);
@@ -57,16 +69,33 @@ __device__ __forceinline__ void boys_fine(double T, const double *__restrict__ t
 #pragma unroll
       for (int m = M - 1; m >= 0; --m) F[m] = fma(t2, F[m + 1], et) * (1.0 / (2 * m + 1));
     }
-  } else {
-    const double rt = rsqrt(T);
-    F[0] = 0.88622692545275801364908374167057 * rt;
-    if (M > 0) {
-      // e^-T is at most 4e-18 here, under 2e-9 of (2m+1) F_m for the orders
-      // of these kernels, so its single-precision value is enough
-      const double et = (double)expf(-(float)T);
-      const double h = 0.5 * rt * rt;
 #pragma unroll
-      for (int m = 0; m < M; ++m) F[m + 1] = fma((double)(2 * m + 1), F[m], -et) * h;
+    for (int n = 0; n <= M; ++n) {
+      F[n] *= s;
+      s *= -2.0 * alpha;
+    }
+  } else {
+    F[0] = 0.88622692545275801364908374167057 * s;
+    if (M > 0) {
+      const double ir = -(A * y2);  // -1 / r2
+      // e^-T in F_{m+1} = ((2m+1) F_m - e^-T) / (2T): at T >= 40 it is below
+      // 3e-17 of F_0, and below 2e-9 of (2m+1) F_m for the orders of these
+      // kernels, so its single-precision value, scaled alike, is enough
+      float ef = 0.f, af = 0.f;
+      if (M > 1) {
+        const float bf = (float)B;
+        af = -2.f * ((float)A / bf);
+        ef = expf(-((float)ar / bf)) * (float)K * rsqrtf(bf) * af;
+      }
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        double v = (double)(2 * m + 1) * F[m];
+        if (m > 0) {
+          v -= (double)ef;
+          ef *= af;
+        }
+        F[m + 1] = v * ir;
+      }
     }
   }
 }
@@ -156,7 +185,11 @@ struct Shape {
   static constexpr int L = LA + LB + LC + LD;
   static constexpr int FB = 2 * LB + 1, FC = 2 * LC + 1, FD = 2 * LD + 1;
   static constexpr int FAx = chunk_most(LA, CA);  // most A functions of a chunk
-  static constexpr int kBlock = L <= 2 ? 256 : L == 3 ? 192 : 256;
+  // Warps against registers: 16 warps of 128 registers up to L = 1, 12 of 168
+  // at L = 2, 8 of 255 above. (H2O)32 / cc-pVDZ with 16 and 12 warps at L = 2
+  // and 3: (ps|ps) 5.0 and 4.4 ms, (pp|ps) 6.9 ms with 12 warps (590 bytes
+  // spilled) and 4.9 ms with 8, (ds|ps) 2.9 and 2.1.
+  static constexpr int kBlock = L <= 1 ? 256 : L == 2 ? 192 : L == 3 ? 128 : 256;
   static constexpr int kMinBlocks = L <= 3 ? 2 : 1;
   static constexpr int kWarps = kBlock / 32;
   static constexpr int kR = row_max_bras(pair_class(LA, LB));  // bras of a segment
@@ -395,18 +428,15 @@ __device__ __forceinline__ void row_body(const JKArgs &a, const double *tab, dou
           double R[n3(L)], ex1[EA], ey1[EA], ez1[EA];
           {
             const double p = w01.x;
-            const double rs = rsqrt(p + q);
-            double alpha = p * q * rs * rs;
-            double s = w45.x * Kk * rs * wgt;
-            erf_attenuate(a.erf_mu2, alpha, s);
+            double A = p * q, B = p + q, K = w45.x * Kk * wgt;
+            if (a.erf_mu2 > 0.0) {
+              B = fma(B, a.erf_mu2, A);
+              A *= a.erf_mu2;
+              K *= sqrt(a.erf_mu2);
+            }
             const double x = w01.y - Qx, y = w23.x - Qy, z = w23.y - Qz;
             double Fs[L + 1];
-            boys_fine<L>(alpha * (x * x + y * y + z * z), tab, Fs);
-#pragma unroll
-            for (int n = 0; n <= L; ++n) {
-              Fs[n] *= s;
-              s *= -2.0 * alpha;
-            }
+            boys_scaled<L>(A, B, x * x + y * y + z * z, K, tab, Fs);
             hermite_r_inplace<L, double>(Fs, x, y, z, R);
             if constexpr (LAB > 0) {
               const double h1 = 0.5 / p;
