@@ -207,7 +207,7 @@ static int grad_impl(dgf_ctx *c, const double *d1, const double *d2, double hfx,
       cudaEventRecord(e0, ls);
     }
     const GradEntry &g = g_grad_entry[cp.X][cp.Y];
-    if (g.row && cp.row_ntask > 0 && nrow < kRowSlots) {
+    if (g.row && (a.spherical || g.row_cart) && cp.row_ntask > 0 && nrow < kRowSlots) {
       a.row_bra = c->d_row_bra + c->cls_off[cp.X];
       a.row_tasks = c->d_row_tasks + cp.row_off;
       a.row_task0 = 0;

@@ -690,6 +690,7 @@ __global__ void __launch_bounds__(128) grad_warp_kernel(const __grid_constant__ 
 typedef void (*PairGradLauncher)(const JKArgs &, const PairGrad &, int grid, cudaStream_t);
 struct GradEntry {
   PairGradLauncher row, warp;
+  bool row_cart;              // the row kernel also takes Cartesian functions
   int row_warps, row_blocks;  // warps per block, resident blocks per SM
   int warp_warps;
   cudaError_t (*prepare)();
@@ -698,11 +699,14 @@ extern GradEntry g_grad_entry[kGradClasses][kGradClasses];  // dgf_grad2e.cu; fi
 
 // Classes with the row kernel: kets (ss) and (ps), where the warp kernel
 // would leave most lanes without a ket component, and (pp) and (ds) kets up to
-// L = 4 (above, a thread's R_tuv and tables spill more than they save, and
-// the unrolled code takes minutes to compile).   On (H2O)9 / cc-pVDZ, warp then
-// row kernel: (ds|pp) 2.88 and 0.15 ms, (pp|pp) 1.45 and 0.17, (ds|ds) 1.00 and
-// 0.08.
+// L = 5 (their larger ones spill R_tuv and take minutes to compile; Cartesian
+// functions stop at L = 4). On (H2O)9 / cc-pVDZ, warp then row kernel: (ds|pp)
+// 2.88 and 0.15 ms, (pp|pp) 1.45 and 0.17, (ds|ds) 1.00 and 0.08, (dp|pp) 1.85
+// and 1.01, (dp|ds) 1.55 and 0.36.
 constexpr bool grad_by_row(int LA, int LB, int LC, int LD) {
+  return ncart(LC) * ncart(LD) <= 3 || LA + LB + LC + LD <= 5;
+}
+constexpr bool grad_by_row_cart(int LA, int LB, int LC, int LD) {
   return ncart(LC) * ncart(LD) <= 3 || LA + LB + LC + LD <= 4;
 }
 // Classes with the warp kernel: the other kets; it also serves the contracted
@@ -712,10 +716,13 @@ constexpr bool grad_by_warp(int LC, int LD) { return ncart(LC) * ncart(LD) > 3; 
 template <int LA, int LB, int LC, int LD>
 void launch_grad_row(const JKArgs &a, const PairGrad &pg, int grid, cudaStream_t s) {
   using R = RowGrad<LA, LB>;
-  if (a.spherical)
-    grad_row_kernel<LA, LB, LC, LD, true><<<grid, R::kBlock, R::smem(), s>>>(a, pg);
-  else
-    grad_row_kernel<LA, LB, LC, LD, false><<<grid, R::kBlock, R::smem(), s>>>(a, pg);
+  if constexpr (grad_by_row_cart(LA, LB, LC, LD)) {
+    if (!a.spherical) {
+      grad_row_kernel<LA, LB, LC, LD, false><<<grid, R::kBlock, R::smem(), s>>>(a, pg);
+      return;
+    }
+  }
+  grad_row_kernel<LA, LB, LC, LD, true><<<grid, R::kBlock, R::smem(), s>>>(a, pg);
 }
 
 template <int LA, int LB, int LC, int LD>
@@ -735,7 +742,8 @@ cudaError_t prepare_grad() {
   };
   if constexpr (grad_by_row(LA, LB, LC, LD)) {
     allow(grad_row_kernel<LA, LB, LC, LD, true>, RowGrad<LA, LB>::smem());
-    allow(grad_row_kernel<LA, LB, LC, LD, false>, RowGrad<LA, LB>::smem());
+    if constexpr (grad_by_row_cart(LA, LB, LC, LD))
+      allow(grad_row_kernel<LA, LB, LC, LD, false>, RowGrad<LA, LB>::smem());
   }
   if constexpr (grad_by_warp(LC, LD)) {
     using W = WarpGrad<LA, LB, LC, LD>;
@@ -752,6 +760,7 @@ void fill_grad() {
   e.prepare = &prepare_grad<LA, LB, LC, LD>;
   if constexpr (grad_by_row(LA, LB, LC, LD)) {
     e.row = &launch_grad_row<LA, LB, LC, LD>;
+    e.row_cart = grad_by_row_cart(LA, LB, LC, LD);
     e.row_warps = RowGrad<LA, LB>::kWarps;
     e.row_blocks = LA + LB + LC + LD <= 1 ? 4 : LA + LB + LC + LD <= 2 ? 3 : 2;
   }
