@@ -1037,15 +1037,18 @@ static void set_row_args(const dgf_ctx *c, const ClassPlan &cp, JKArgs &a, int t
 // of at most R bras of one A shell, each with the 32-ket chunks its longest
 // prefix reaches, at most G chunks a task: {first bra, bras | chunks << 16,
 // first ket, end of the kets}.  R starts at max_bras and is halved while that
-// leaves fewer segment-chunks than about one per resident warp of the GPU (a
-// segment's tile then has fewer bras to spread its own atomics over, but a
-// small molecule would leave most warps without work); G, at most 16, leaves
-// every warp several tasks.  min_width < 32 (pack kernels, whose warps work
+// leaves too few segment-chunks for the GPU (a segment's tile then has fewer
+// bras to spread its own atomics over); G, at most 16, leaves every warp
+// several tasks.  min_width < 32 (pack kernels, whose warps work
 // through a chunk's kets one after the other): chunks too are halved, down to
 // that, while there are too few.  Depends on the molecules and the threshold only,
 // so that every rank of a sharded build makes the same list.
 void row_tasks(const std::vector<RowSource> &src, int max_bras, int min_width, std::vector<int4> &tasks) {
-  const int64_t units_want = 148 * 10, tasks_want = 148 * 12 * 4;
+  // (H2O)4 / cc-pVDZ took 580, 440 and 380 us with 1480, 740 and 296 wanted
+  // segment-chunks of a row launch, (H2O)32 the same within 1%: the class
+  // launches run beside each other, and longer tiles mean fewer atomics.  A
+  // pack kernel's task is one warp's serial work: 2960.
+  const int64_t units_want = min_width < 32 ? 148 * 20 : 148 * 2, tasks_want = 148 * 12 * 4;
   int width = 32;
   auto segments = [&](int R, auto f) {
     for (const RowSource &s : src)
@@ -2011,7 +2014,6 @@ extern "C" int dgf_autotune(dgf_ctx *c, const double *dmat_device, const dgf_opt
   DGF_CUDA_CHECK(cudaEventCreate(&e1));
   std::string rep = "[";
   ++c->gen;
-  c->user_tuned = true;
   c->row_slot = kRowSlots;  // the first row launch clears the task counters
   const int saved_prof = c->profiling;
   c->profiling = 0;

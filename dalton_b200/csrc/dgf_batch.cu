@@ -135,9 +135,8 @@ extern "C" int dgf_batch_create(dgf_ctx *const *caller_ctxs, dgf_int nmol, dgf_b
   if (!caller_ctxs || nmol <= 0) BFAIL(DGF_ERR_ARG, "empty batch");
   for (dgf_int m = 0; m < nmol; ++m)
     if (!caller_ctxs[m]) BFAIL(DGF_ERR_ARG, "NULL context in batch");
-  // Contracted contexts take part in their resolved form where all of them
-  // have it (one tuned context keeps the batch contracted: its choices are
-  // for the contracted classes).
+  // Contracted contexts take part in their resolved form, unless a kernel was
+  // pinned on one of them (its choices are for the contracted classes).
   std::vector<dgf_ctx *> ctxs(caller_ctxs, caller_ctxs + nmol);
   bool tuned = false, resolved = false;
   for (dgf_ctx *c : ctxs) tuned = tuned || c->user_tuned;

@@ -74,7 +74,7 @@ struct dgf_ctx {
   // from the copy of the basis kept here.
   bool resolve_all = false;   // this is such a second context
   bool prim_fits = false;     // the resolved form exists and fits every entry point
-  bool user_tuned = false;    // kernel choices were made for this context: it serves all calls itself
+  bool user_tuned = false;    // a kernel was pinned on this context: it serves all calls itself
   dgf_ctx *prim = nullptr;
   dgf_basis basis_copy = {};
   std::vector<dgf_int> basis_i;
@@ -185,7 +185,7 @@ void row_tasks(const std::vector<RowSource> &src, int max_bras, int min_width, s
 // one (relative), where the contracted form drops nothing.
 constexpr double kPrimThrs = 1e-3;
 // The context a direct build or gradient of `c` runs in: its resolved form
-// when it has one and nothing was tuned on `c`, else itself (dgf_api.cu).
+// when it has one and no kernel was pinned on `c`, else itself (dgf_api.cu).
 dgf_ctx *direct_ctx(dgf_ctx *c);
 
 // The single-molecule form of the AO <-> working-basis maps of a context.

@@ -78,7 +78,9 @@ extern "C" int dgf_fock_device_noalloc(dgf_ctx *c, const double *dmat_device, do
     return fail(DGF_ERR_ARG, __LINE__,
                 "dgf_fock_device_noalloc: " + std::to_string(c->nbf) + " basis functions exceed its fixed scratch (" +
                     std::to_string(kNoAllocMaxN) + " at most); use dgf_fock_device");
-  if (c->prim && direct_ctx(c) == c->prim) {  // where the caller's dgf_fock calls made their plan
+  // the caller's dgf_fock calls made their plan in the resolved context, a
+  // store or the autotuner in this one
+  if (c->prim && direct_ctx(c) == c->prim && !c->prim->plan.empty() && c->prim->plan_thrs == thrs * kPrimThrs) {
     c = c->prim;
     thrs *= kPrimThrs;
   }
