@@ -59,29 +59,41 @@ def class_flops(la, lb, lc, ld, prim_quartets, quartets, spherical=True) -> floa
                                                                                                    spherical)
 
 
-# Two-electron gradient (backward kernel), one fixed count per class:
-# per primitive quartet the Boys function and R_tuv to L+1, and for each of
-# the three differentiated centres (A, B, C; D by translational invariance)
-# and each direction the ket and bra contractions with that centre's angular
-# momentum raised by one; per contracted quartet the density product (8 flops
-# per Cartesian integral) and its contraction with the nine derivative
-# blocks (2 flops each).
+# Two-electron gradient in relative coordinates, one fixed count per class:
+# per primitive quartet the Boys function and R_tuv to L+1 and, for each ket
+# component, its transform to Hermite indices up to Lab+1, the contraction of
+# the density product with the bra coefficients and with the lowered ones of
+# each direction, the energy and the three dE/dP sums, and the three sums over
+# lowered ket coefficients; per contracted quartet the density product (16
+# flops per Cartesian integral).  Coefficient ranges are those of the
+# components (t <= i + j in each direction).
+def _cart(l):
+    return [(x, y, l - x - y) for x in range(l, -1, -1) for y in range(l - x, -1, -1)]
+
+
+def _ranges(l1, l2):
+    """For each component pair: the number of Hermite indices, and their
+    number with one direction lowered, summed over the directions."""
+    out = []
+    for c in _cart(l1):
+        for d in _cart(l2):
+            s = [c[k] + d[k] + 1 for k in range(3)]
+            full = s[0] * s[1] * s[2]
+            out.append((full, sum(full // s[k] * (s[k] - 1) for k in range(3))))
+    return out
+
+
 def grad_flops_per_primitive(la, lb, lc, ld) -> float:
-    L = la + lb + lc + ld + 1
+    L, lab = la + lb + lc + ld + 1, la + lb
     f = 40 + 3 * L + 3 * sum(n3(j) for j in range(1, L + 1))
-    for centre in range(3):
-        ls = [la, lb, lc, ld]
-        ls[centre] += 1
-        lab, lcd = ls[0] + ls[1], ls[2] + ls[3]
-        ket = 2 * n3(lab) * n3(lcd) * ncart(ls[2]) * ncart(ls[3])
-        bra = 2 * n3(lab) * ncart(ls[0]) * ncart(ls[1]) * ncart(ls[2]) * ncart(ls[3])
-        f += 3 * (ket + bra)
+    bra = sum(2 * full + 2 * low for full, low in _ranges(la, lb))
+    for full, low in _ranges(lc, ld):
+        f += 2 * full * n3(lab + 1) + bra + 8 * n3(lab) + 2 * low * n3(lab)
     return float(f)
 
 
 def grad_flops_per_contracted(la, lb, lc, ld) -> float:
-    ncart4 = ncart(la) * ncart(lb) * ncart(lc) * ncart(ld)
-    return float(8 * ncart4 + 2 * 9 * ncart4)
+    return float(16 * ncart(la) * ncart(lb) * ncart(lc) * ncart(ld))
 
 
 def grad_class_flops(la, lb, lc, ld, prim_quartets, quartets) -> float:
