@@ -231,6 +231,19 @@ static int class_route(const dgf_ctx *c, const ClassPlan &cp, int nslot, bool sh
   return row ? kRouteRow : kRouteOther;
 }
 
+// Whether an FP64 build of several density slots launches the row kernel of an
+// entry once per slot, which forms the integrals anew for each, in place of the
+// thread kernel that digests all slots in one pass: where the entry gives the
+// resident warps' lanes two quartets each (148 SMs, 8 warps), or the caller
+// pinned the row kernel. With seven slots in cc-pVDZ, thread kernels then rows
+// throughout: H2O 0.30 and 0.38 ms (launches that fill no SM), (H2O)2 0.54 and
+// 0.59, (H2O)3 1.13 both, (H2O)5 4.13 and 3.19, (H2O)10 19.9 and 13.7; with
+// this rule 0.28, 0.51, 1.01, 3.12 and 13.3.
+static bool row_per_slot(const dgf_ctx *c, const ClassPlan &cp, bool sharded) {
+  if (class_route(c, cp, 1, sharded) != kRouteRow) return false;
+  return cp.nquartet >= 148 * 8 * 32 * 2 || (!sharded && c->choice[cp.X][cp.Y][0] == kRowVariant);
+}
+
 // Whether the mixed form splits an untuned class although a pack kernel has it.
 static bool keeps_split(const dgf_ctx *c, const ClassPlan &cp, int route) {
   return route == kRoutePack && c->split_ok[cp.X][cp.Y] == 1 && pair_l(cp.X) + pair_l(cp.Y) >= 7;
@@ -1574,6 +1587,8 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
     struct Item {
       size_t e;
       int pass;
+      int slot;  // the one slot of a row launch among several, or -1: all of them
+      bool first;  // of the item's entry and pass: this launch counts its quartets
       double s;  // estimated time
     };
     std::vector<Item> items;
@@ -1588,7 +1603,18 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
         // model operations at 5 TFLOP/s, plus the time one quartet takes alone
         const double t = (double)(sq1[e] - sq0[e]) * entry_cost_per_quartet(c, c->plan[e]) / 5e12 + 6e-6 +
                          2e-7 * n3(pair_l(c->plan[e].X) + pair_l(c->plan[e].Y));
-        items.push_back({e, pass, t});
+        if (ns > 1 && !stored && o.mixed_cutoff <= 0.0 && row_per_slot(c, c->plan[e], o.shard_count > 1)) {
+          bool first = true;
+          for (int s = 0; s < ns; ++s) {
+            const SlotSpec &sp = slots[s0 + s];
+            if (pass == 0 ? sp.js == 0.0 && sp.ks == 0.0 : sp.ka == 0.0) continue;
+            items.push_back({e, pass, s, first, t});
+            first = false;
+            seconds += t;
+          }
+          continue;
+        }
+        items.push_back({e, pass, -1, true, t});
         seconds += t;
       }
     }
@@ -1621,6 +1647,21 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
         set_row_args(c, cp, ra, t0, t1);
       };
       auto counters = [&]() { return count ? c->d_cnt + 4 * (nlaunch_class % kCounterSlots) : nullptr; };
+      if (it.slot >= 0) {
+        JKArgs ra = a;
+        ra.nslot = 1;
+        ra.D += it.slot * n2;
+        ra.Ds += it.slot * n2;
+        ra.Fh += it.slot * n2;
+        if (ra.blk_dmax_slot) ra.blk_dmax_slot += it.slot * nb2;
+        ra.jscale[0] = a.jscale[it.slot];
+        ra.kscale[0] = a.kscale[it.slot];
+        set_task_range(ra);
+        ra.counters = it.first ? counters() : nullptr;
+        ++nlaunch_class;
+        ++launches;
+        return launch_kernel(c, jk_row_entry(cp.X, cp.Y), cp.X, cp.Y, ra, ls, 0);
+      }
       if (stored) {  // conventional form: digest the stored blocks
         a.store_in = c->d_store;
         a.store_base = c->store_off[e];

@@ -28,8 +28,9 @@ struct ClassPlan {
   int64_t row_off = 0;
   int row_ntask = 0;
 };
-// Task counters of the row launches of a call (kRowChunksMax each).
-constexpr int kRowSlots = 128;
+// Task counters of the row launches of a call (kRowChunksMax each): at most 55
+// plan entries, eight density slots, two operators.
+constexpr int kRowSlots = 1024;
 
 // Map between the AO basis (Dalton's contracted functions) and the
 // two-electron working basis, as sparse rows: wr_* gives, for every working

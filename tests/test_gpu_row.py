@@ -103,7 +103,7 @@ def test_default_kernels_match_oracle(cuda, orc, name):
 @pytest.mark.parametrize("name", ["h2o3_dz", "c2h6_tz"])
 def test_several_densities(cuda, name):
     """More than one density slot: the pack kernels digest the slots one after
-    the other, the row classes fall back; against one build per density."""
+    the other, the row classes launch once per slot; against one build per density."""
     mol, basis = MOLS[name]
     bs = build_basis(mol(), basis)
     fb = FockBuilder(bs)
@@ -114,6 +114,28 @@ def test_several_densities(cuda, name):
     for k in range(9):
         g = fb.herfck(d[k], ift[k])
         assert np.abs(f[k] - g).max() < 1e-15 * bs.nbf * max(1.0, np.abs(g).max())
+
+
+@pytest.mark.parametrize("name", ["h2o3_dz", "h2o2_aug", "c2h6_tz"])
+def test_several_densities_by_slot(cuda, name):
+    """Several slots through the row kernels, one launch per slot, against the
+    thread kernels that take all slots at once: screens over all densities,
+    slots without Coulomb or exchange part, the attenuated pass, the counts."""
+    mol, basis = MOLS[name]
+    bs = build_basis(mol(), basis)
+    fb, ft = FockBuilder(bs), FockBuilder(bs)
+    _pin(fb, -5)
+    for v in (-5, -6):
+        _pin(ft, v, 0)
+    scale = np.array([1.0, 1e-3, 1.0, 1e-2, 1.0])[:, None, None] * 0.1
+    d = np.random.default_rng(12).normal(size=(5, bs.nbf, bs.nbf)) * scale
+    ift = [3, 13, 22, 11, 12]
+    for o in ({}, {"hfxfac": 0.0}, {"hfxfac": 0.3}, {"ifthrs": 9, "icedif": 0}, {"hfxmu": 0.5, "hfxatt": 0.4}):
+        f, g = fb.herfck(d, ift, **o), ft.herfck(d, ift, **o)
+        for key in ("quartets_total", "quartets_skipped", "prim_quartets"):
+            assert fb.last_stats[key] == ft.last_stats[key], (o, key)
+        # another order of summation of up to nbf^2 terms of the matrices' size
+        assert np.abs(f - g).max() < 1e-15 * bs.nbf * max(1.0, np.abs(g).max()), o
 
 
 @pytest.mark.parametrize("nshard", [2, 5])
