@@ -215,9 +215,10 @@ static bool row_ok(const dgf_ctx *c, const ClassPlan &cp) {
   return cp.row_ntask > 0 && sph && c->d_ks_i && c->nwf <= 46340 && jk_row_entry(cp.X, cp.Y).launch;
 }
 
-// The pack kernel: spherical functions, pair fragments made.
+// The pack kernel: spherical functions, pair fragments made (a sharded build
+// fails where they could not be).
 static bool pack_ok(const dgf_ctx *c, const ClassPlan &cp) {
-  return cp.row_ntask > 0 && c->spherical && g_pack_table[cp.X][cp.Y].launch && c->d_frag[cp.X] && c->d_frag[cp.Y];
+  return cp.row_ntask > 0 && c->pack_on && c->spherical && g_pack_table[cp.X][cp.Y].launch && c->d_frag[cp.X] && c->d_frag[cp.Y];
 }
 
 enum { kRouteOther = 0, kRouteRow = 1, kRoutePack = 2 };
@@ -740,14 +741,20 @@ static void keep_basis(dgf_ctx *c, const dgf_basis *b) {
 
 static int create_ctx(const dgf_basis *b, int device, bool resolve_all, dgf_ctx **out);
 
-dgf_ctx *direct_ctx(dgf_ctx *c) {
-  if (!c->prim_fits || c->user_tuned) return c;
-  if (!c->prim && create_ctx(&c->basis_copy, c->device, true, &c->prim) != DGF_OK) {
-    c->prim = nullptr;  // no memory for it: the contracted form serves
-    c->prim_fits = false;
-    return c;
+int direct_ctx(dgf_ctx *c, bool sharded, dgf_ctx **out) {
+  *out = c;
+  if (!c->prim_fits || (!sharded && (c->user_tuned || c->prim_failed))) return DGF_OK;
+  if (!c->prim) {
+    const int r = create_ctx(&c->basis_copy, c->device, true, &c->prim);
+    c->prim_failed = r != DGF_OK;
+    if (r) {
+      c->prim = nullptr;
+      cudaGetLastError();
+      return sharded ? r : DGF_OK;
+    }
   }
-  return c->prim;
+  *out = c->prim;
+  return DGF_OK;
 }
 
 extern "C" int dgf_create(const dgf_basis *b, int device, dgf_ctx **out) { return create_ctx(b, device, false, out); }
@@ -1104,22 +1111,33 @@ static int launch_pack(dgf_ctx *c, const ClassPlan &cp, JKArgs &a, cudaStream_t 
 }
 
 // Pair fragments of the classes the plan's pack kernels read, once per
-// context.  Without the memory for them the classes keep their other kernels.
+// context.  Above their bound, which depends on the plan alone, or without the
+// memory for them (frag_short) the classes keep their other kernels.
 static int ensure_frags(dgf_ctx *c, const std::vector<ClassPlan> &plan) {
+  c->pack_on = c->frag_short = false;
   if (!c->spherical) return DGF_OK;
   bool need[kNumPairClass] = {}, made = false;
   for (const ClassPlan &cp : plan)
     if (cp.row_ntask > 0 && g_pack_table[cp.X][cp.Y].launch) need[cp.X] = need[cp.Y] = true;
-  size_t total = 0;
-  for (int X = 0; X < kNumPairClass; ++X)
-    if (need[X] || c->d_frag[X]) total += (size_t)(c->cls_off[X + 1] - c->cls_off[X]) * g_frag_table[X].doubles * 8;
+  size_t total = 0, kept = 0;  // of this plan, and of earlier plans only
+  for (int X = 0; X < kNumPairClass; ++X) {
+    const size_t bytes = (size_t)(c->cls_off[X + 1] - c->cls_off[X]) * g_frag_table[X].doubles * 8;
+    if (need[X]) total += bytes;
+    else if (c->d_frag[X]) kept += bytes;
+  }
   if (total > kFragMaxBytes) return DGF_OK;
+  c->pack_on = true;
   for (int X = 0; X < kNumPairClass; ++X) {
     const int n = c->cls_off[X + 1] - c->cls_off[X];
+    if (!need[X] && c->d_frag[X] && total + kept > kFragMaxBytes) {
+      cudaFree(c->d_frag[X]);
+      c->d_frag[X] = nullptr;
+    }
     if (!need[X] || c->d_frag[X] || !n) continue;
     if (dev_alloc(&c->d_frag[X], (size_t)n * g_frag_table[X].doubles) != cudaSuccess) {
       cudaGetLastError();
       c->d_frag[X] = nullptr;
+      c->frag_short = true;
       continue;
     }
     g_frag_table[X].launch(c->d_pairs + c->cls_off[X], c->d_pp, n, c->d_sph, c->d_frag[X],
@@ -1509,6 +1527,12 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
   }
   int st_code = build_plan(c, o.thrs);
   if (st_code) return st_code;
+  if (o.shard_count > 1 && c->frag_short) {  // every rank has to run the pack kernels
+    ++c->gen;
+    st_code = ensure_frags(c, c->plan);
+    if (st_code) return st_code;
+    if (c->frag_short) DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the pair fragments failed; a shard needs them");
+  }
   // Density screening as Dalton's direct Fock build: on when IFTHRS < 16,
   // IFTHRS < 4 taken as 14 (DALTON/abacus/her2drv.F:520-540).
   int64_t ifthrs = o.ifthrs;
@@ -1825,7 +1849,8 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
 // A direct build of c, in its resolved context where there is one.
 static int fock_direct(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double *dmat_dev, double *fmat_dev,
                        const dgf_options *opt, cudaStream_t st, dgf_stats *stats) {
-  dgf_ctx *d = direct_ctx(c);
+  dgf_ctx *d = nullptr;
+  if (const int r = direct_ctx(c, opt && opt->shard_count > 1, &d)) return r;
   if (d == c) return fock_impl(c, ndmat, ifctyp, dmat_dev, fmat_dev, opt, st, stats);
   dgf_options o;
   dgf_default_options(&o);

@@ -142,7 +142,8 @@ extern "C" int dgf_batch_create(dgf_ctx *const *caller_ctxs, dgf_int nmol, dgf_b
   for (dgf_ctx *c : ctxs) tuned = tuned || c->user_tuned;
   if (!tuned)
     for (dgf_ctx *&c : ctxs) {
-      dgf_ctx *d = direct_ctx(c);
+      dgf_ctx *d = nullptr;
+      if (const int r = direct_ctx(c, false, &d)) return r;
       resolved = resolved || d != c;
       c = d;
     }

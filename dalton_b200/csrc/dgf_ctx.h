@@ -74,8 +74,9 @@ struct dgf_ctx {
   // builds and gradients use (direct_ctx).  It is made by the first of them
   // from the copy of the basis kept here.
   bool resolve_all = false;   // this is such a second context
-  bool prim_fits = false;     // the resolved form exists and fits every entry point
-  bool user_tuned = false;    // a kernel was pinned on this context: it serves all calls itself
+  bool prim_fits = false;     // the basis has a resolved form that fits every entry point
+  bool prim_failed = false;   // it could not be made here (no memory): this context serves the whole builds
+  bool user_tuned = false;    // a kernel was pinned on this context: it serves all calls itself, shards excepted
   dgf_ctx *prim = nullptr;
   dgf_basis basis_copy = {};
   std::vector<dgf_int> basis_i;
@@ -122,6 +123,8 @@ struct dgf_ctx {
   int4 *d_row_tasks = nullptr;
   size_t row_tasks_cap = 0;
   double *d_frag[dgf::kNumPairClass] = {};  // pack kernels: the classes' pair fragments, made with the first plan that uses them
+  bool pack_on = false;     // the plan's fragments stay within their bound
+  bool frag_short = false;  // ... but there was no memory for some of them
   unsigned *d_row_work = nullptr;
   int row_slot = 0;  // next free slot of d_row_work in the running call
   // per-call buffers
@@ -185,9 +188,12 @@ void row_tasks(const std::vector<RowSource> &src, int max_bras, int min_width, s
 // threshold the Fock matrix of H2O / 6-31G* was 2e-13 from the unscreened
 // one (relative), where the contracted form drops nothing.
 constexpr double kPrimThrs = 1e-3;
-// The context a direct build or gradient of `c` runs in: its resolved form
-// when it has one and no kernel was pinned on `c`, else itself (dgf_api.cu).
-dgf_ctx *direct_ctx(dgf_ctx *c);
+// The context a direct build or gradient of `c` runs in (dgf_api.cu): its
+// resolved form when it has one, can be made, and no kernel was pinned on `c`;
+// else itself.  A shard's context depends on the basis alone, as all ranks
+// must cut the same queue: pins do not count, and where the resolved form
+// cannot be made the call fails.
+int direct_ctx(dgf_ctx *c, bool sharded, dgf_ctx **out);
 
 // The single-molecule form of the AO <-> working-basis maps of a context.
 inline dgf::WorkMaps ctx_maps(const dgf_ctx *c) {

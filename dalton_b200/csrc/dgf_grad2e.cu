@@ -264,7 +264,8 @@ static int grad_impl(dgf_ctx *c, const double *d1, const double *d2, double hfx,
 // The gradient in the resolved context of c where there is one.
 static int grad_direct(dgf_ctx *c, const double *d1, const double *d2, double hfx, double thrs, double *grad,
                        cudaStream_t st) {
-  dgf_ctx *d = direct_ctx(c);
+  dgf_ctx *d = nullptr;
+  if (const int r = direct_ctx(c, false, &d)) return r;
   if (d == c) return grad_impl(c, d1, d2, hfx, thrs, grad, st);
   d->profiling = c->profiling;
   const int r = grad_impl(d, d1, d2, hfx, thrs * kPrimThrs, grad, st);

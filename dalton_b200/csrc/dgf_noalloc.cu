@@ -80,7 +80,7 @@ extern "C" int dgf_fock_device_noalloc(dgf_ctx *c, const double *dmat_device, do
                     std::to_string(kNoAllocMaxN) + " at most); use dgf_fock_device");
   // the caller's dgf_fock calls made their plan in the resolved context, a
   // store or the autotuner in this one
-  if (c->prim && direct_ctx(c) == c->prim && !c->prim->plan.empty() && c->prim->plan_thrs == thrs * kPrimThrs) {
+  if (c->prim && !c->user_tuned && !c->prim->plan.empty() && c->prim->plan_thrs == thrs * kPrimThrs) {
     c = c->prim;
     thrs *= kPrimThrs;
   }

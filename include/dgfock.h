@@ -105,7 +105,12 @@ typedef struct {
    * range shard_index is evaluated, as Dalton's parallel Fock build hands
    * cost-sorted shell-pair tasks to its workers (herpar.F:457,1165); F is
    * then the partial sum of that shard (sum the shards, e.g. with an NCCL
-   * all-reduce, for the full matrix).  0 and 1 = everything. */
+   * all-reduce, for the full matrix).  The shards of one matrix are the same
+   * call on contexts of the same basis, but for shard_index; how a context
+   * was tuned or pinned before does not move its cut points, and the kernels
+   * of a shard are the classes' defaults.  Where a rank cannot allocate what
+   * the others' shards use, its call fails (DGF_ERR_NOMEM, DGF_ERR_CUDA).
+   * 0 and 1 = everything. */
   dgf_int shard_index;
   dgf_int shard_count;
   /* ICEDIF (HR2INP .ICEDIF, DALTON/abacus/herdrv.F:2042-2044,2131): with

@@ -152,6 +152,25 @@ def test_row_shards_tile(cuda, nshard):
     assert np.abs(f - ref).max() < 1e-12 * max(1.0, np.abs(ref).max())
 
 
+@pytest.mark.parametrize("basis", ["6-31G*", "cc-pVTZ"])
+def test_shards_tile_with_a_pinned_rank(cuda, basis):
+    """The same in a segmented basis, whose whole builds run in the contracted
+    form once a kernel is pinned, and with the pack kernels of f shells: one
+    rank pinned, one autotuned, one with a copied tuning, the others as made."""
+    import torch
+
+    bs = build_basis(molecules.water_cluster(2, seed=4), basis)
+    d = _density(bs.nbf, 5)
+    ref = FockBuilder(bs).herfck(d, 13)
+    fbs = [FockBuilder(bs) for _ in range(5)]
+    fbs[0].set_class_kernel((1, 0, 0, 0), 0)
+    fbs[1].autotune(torch.tensor(d, device=cuda))
+    fbs[2].copy_tuning_from(fbs[0])
+    f = sum(fb.herfck(d, 13, shard=(r, 5)) for r, fb in enumerate(fbs))
+    # every quartet in one shard: only the order of the sums differs
+    assert np.abs(f - ref).max() < 1e-15 * bs.nbf * max(1.0, np.abs(ref).max())
+
+
 def test_graph_replay(cuda):
     """Repeated short builds (replayed as graphs from the second call on):
     new densities, buffers, streams and options between the calls, plan and

@@ -1,0 +1,141 @@
+"""Host paths of libdgfock that decide which quartets a call evaluates, and
+what it does when a CUDA call fails, on a CUDA runtime without a GPU
+(fake_cudart.cpp, preloaded in a child process): kernels do not run, their
+launches are checked against the live allocations and the quartets that they
+cover are counted."""
+import json
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+PRELUDE = """
+import ctypes, json, os, sys
+sys.path.insert(0, {root!r})
+import numpy as np
+from dalton_b200 import _lib, molecules
+from dalton_b200.basis import build_basis
+from dalton_b200.fock import FockBuilder
+
+F = ctypes.CDLL({fake!r})
+F.fake_kernels.restype = F.fake_bad.restype = ctypes.c_char_p
+for n in ("fake_quartets", "fake_not_once", "fake_launches", "fake_replays", "fake_streams", "fake_live", "fake_malloc_calls"):
+    getattr(F, n).restype = ctypes.c_long
+F.fake_fail_malloc.argtypes = [ctypes.c_long] * 2
+
+def builder(basis, n=1):
+    return FockBuilder(build_basis(molecules.water_cluster(n, seed=2), basis))
+
+def status(f, *a, **k):
+    try:
+        f(*a, **k)
+    except _lib.DgfError as e:
+        return e.status
+    return 0
+
+def covered(f=None):
+    if f is not None:
+        F.fake_reset()
+        f()
+    return dict(quartets=F.fake_quartets(), not_once=F.fake_not_once(), bad=F.fake_bad().decode(),
+                kernels=F.fake_kernels().decode().split())
+
+def eye(fb):
+    return np.eye(fb.nbf)
+
+def out(**kw):
+    print("RESULT " + json.dumps(kw))
+"""
+
+
+@pytest.fixture(scope="session")
+def host(tmp_path_factory):
+    """Runs a snippet in a child with the fake runtime; returns its result."""
+    lib = str(tmp_path_factory.mktemp("fake") / "libfakecudart.so")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "dalton_b200", "csrc"),
+                    "-I", os.path.join(ROOT, "include"), "-I", "/usr/local/cuda/include",
+                    os.path.join(HERE, "fake_cudart.cpp"), "-o", lib], check=True)
+
+    def run(code):
+        src = PRELUDE.format(root=ROOT, fake=lib) + textwrap.dedent(code)
+        r = subprocess.run([sys.executable, "-c", src], env=dict(os.environ, LD_PRELOAD=lib), capture_output=True,
+                           text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        return json.loads([ln for ln in r.stdout.splitlines() if ln.startswith("RESULT ")][-1][7:])
+
+    return run
+
+
+SHARDS = """
+basis, n = {basis!r}, 3
+whole = covered(lambda: builder(basis).herfck(eye(builder(basis)), thrs=1e-6))
+fbs = [builder(basis) for _ in range(n)]
+{setup}
+F.fake_reset()
+got = [status(fb.herfck, eye(fb), thrs=1e-6, shard=(r, n)) for r, fb in enumerate(fbs)]
+out(whole=whole, got=got, parts=covered())
+"""
+
+
+@pytest.mark.parametrize("basis", ["cc-pVDZ", "6-31G*", "STO-3G", "cc-pVTZ"])
+@pytest.mark.parametrize("state", ["alike", "pinned", "copied", "stored"])
+def test_shards_tile_whatever_a_rank_did_before(host, basis, state):
+    """The shards of one build cover every quartet once, also where one
+    rank's context was pinned to other kernels, took over such a tuning, or
+    holds an integral store: none of these may move its cut points."""
+    setup = {"alike": "", "pinned": "fbs[0].set_class_kernel((1, 0, 0, 0), 0)",
+             "copied": "p = builder(basis); p.set_class_kernel((1, 0, 1, 0), 0); fbs[0].copy_tuning_from(p)",
+             "stored": "_lib.check(_lib.load().dgf_store_integrals(fbs[0]._h, 1e-6, 0, None, None), 'store')"}[state]
+    r = host(SHARDS.format(basis=basis, setup=setup))
+    assert r["got"] == [0, 0, 0]
+    assert r["parts"]["quartets"] == r["whole"]["quartets"] and r["parts"]["not_once"] == 0
+    assert r["parts"]["bad"] == ""
+
+
+@pytest.mark.parametrize("basis", ["6-31G*", "cc-pVTZ"])
+def test_shard_without_memory_is_an_error(host, basis):
+    """A rank that cannot allocate what the others' shards use (the resolved
+    context of a segmented basis, the pair fragments of the pack kernels)
+    reports it instead of cutting the queue another way, and builds its shard
+    once there is memory; a whole build goes on with what it has.  One
+    allocation of a first build fails, or a run of them."""
+    r = host(f"""
+    basis, n = {basis!r}, 2
+    other = builder(basis)
+    d = eye(other)
+    whole = covered(lambda: other.herfck(d, thrs=1e-6))
+    fb = builder(basis)
+    calls = F.fake_malloc_calls()
+    fb.herfck(d, thrs=1e-6, shard=(0, n))
+    calls = F.fake_malloc_calls() - calls
+    sharded, alone = [], []
+    for k, fails in [(k, m) for k in range(calls) for m in (1, 6)]:
+        for shard, res in ((n, sharded), (1, alone)):
+            fb = builder(basis)
+            F.fake_reset()
+            F.fake_fail_malloc(k, fails)
+            s = status(fb.herfck, d, thrs=1e-6, shard=(0, shard))
+            F.fake_fail_malloc(0, 0)
+            why = _lib.last_error() if s else ''
+            if s:
+                F.fake_reset()
+                assert status(fb.herfck, d, thrs=1e-6, shard=(0, shard)) == 0
+            if shard > 1:
+                other.herfck(d, thrs=1e-6, shard=(1, n))
+            c = covered()
+            res.append([s, c["quartets"] - whole["quartets"], c["not_once"], c["bad"], why])
+    out(sharded=sharded, alone=alone)
+    """)
+    if basis == "6-31G*":
+        assert any(s[0] and not a[0] for s, a in zip(r["sharded"], r["alone"]))
+    assert any("pair fragments" in s[4] for s in r["sharded"])
+    assert not any("pair fragments" in a[4] for a in r["alone"])
+    for s, missing, not_once, bad, _ in r["sharded"]:
+        assert s in (0, 2, 3) and (missing, not_once, bad) == (0, 0, ""), r["sharded"]
+    for s, missing, not_once, bad, _ in r["alone"]:
+        assert s in (0, 2, 3) and (not_once, bad) == (0, ""), r["alone"]
