@@ -1202,11 +1202,11 @@ static int build_plan(dgf_ctx *c, double thrs) {
         }
       }
     }
+  c->plan.clear();  // its buffers are replaced below: a failure on the way leaves no plan
   if (tasks.size() > c->row_tasks_cap) {
     if (c->d_row_tasks) cudaFree(c->d_row_tasks);
     c->d_row_tasks = nullptr;
     c->row_tasks_cap = 0;
-    c->plan.clear();
     if (dev_alloc(&c->d_row_tasks, tasks.size()) != cudaSuccess) {
       cudaGetLastError();
       DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the row tasks failed");

@@ -428,6 +428,15 @@ static int batch_plan(dgf_batch *b, double thrs) {
           kbase.resize(bp.koff);
         }
       }
+  // the plan's buffers are replaced: a failure on the way leaves no plan, and
+  // no captured graph of the old one
+  b->plan.clear();
+  if (b->exec) {
+    cudaGraphExecDestroy(b->exec);
+    cudaGraphDestroy(b->graph);
+    b->exec = nullptr;
+    b->graph = nullptr;
+  }
   if (b->d_qoff) cudaFree(b->d_qoff);
   if (b->d_kbase) cudaFree(b->d_kbase);
   if (b->d_row_tasks) cudaFree(b->d_row_tasks);
@@ -437,7 +446,6 @@ static int batch_plan(dgf_batch *b, double thrs) {
   if (!tasks.empty()) {
     if (cudaMalloc(&b->d_row_tasks, tasks.size() * sizeof(int4)) != cudaSuccess) {
       cudaGetLastError();
-      b->plan.clear();
       BFAIL(DGF_ERR_NOMEM, "device allocation of the batch plan failed");
     }
     if (cudaMemcpy(b->d_row_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -453,12 +461,6 @@ static int batch_plan(dgf_batch *b, double thrs) {
     BFAIL(DGF_ERR_CUDA, "upload of the batch plan failed");
   b->plan.swap(plan);
   b->plan_thrs = thrs;
-  if (b->exec) {  // a captured graph refers to the old plan
-    cudaGraphExecDestroy(b->exec);
-    cudaGraphDestroy(b->graph);
-    b->exec = nullptr;
-    b->graph = nullptr;
-  }
   return DGF_OK;
 }
 

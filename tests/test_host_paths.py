@@ -139,3 +139,73 @@ def test_shard_without_memory_is_an_error(host, basis):
         assert s in (0, 2, 3) and (missing, not_once, bad) == (0, 0, ""), r["sharded"]
     for s, missing, not_once, bad, _ in r["alone"]:
         assert s in (0, 2, 3) and (not_once, bad) == (0, ""), r["alone"]
+
+
+@pytest.mark.parametrize("basis", ["cc-pVDZ", "cc-pVTZ", "6-31G*"])
+def test_failed_plan_does_not_stay(host, basis):
+    """A build whose plan for another threshold could not be made leaves
+    nothing behind that a later build would read: each allocation of the
+    second threshold's build fails once, then the first threshold's build and
+    the second's are made again."""
+    r = host(f"""
+    basis = {basis!r}
+    a, b = 1e-2, 1e-7
+    ref = builder(basis)
+    d = eye(ref)
+    whole = [covered(lambda: ref.herfck(d, thrs=t)) for t in (a, b)]
+    fb = builder(basis)
+    fb.herfck(d, thrs=a)
+    calls = F.fake_malloc_calls()
+    fb.herfck(d, thrs=b)
+    calls = F.fake_malloc_calls() - calls
+    res = []
+    for k in range(calls):
+        fb = builder(basis)
+        for _ in range(3):
+            fb.herfck(d, thrs=a)
+        F.fake_fail_malloc(k, 1)
+        s = status(fb.herfck, d, thrs=b)
+        F.fake_fail_malloc(0, 0)
+        for t, w in zip((a, a, b), (whole[0], whole[0], whole[1])):
+            c = covered(lambda: fb.herfck(d, thrs=t))
+            res.append([k, s, c["quartets"] - w["quartets"], c["not_once"], c["bad"]])
+    out(res=res)
+    """)
+    assert any(s for _, s, *_ in r["res"])
+    for k, s, missing, not_once, bad in r["res"]:
+        assert (missing, not_once, bad) == (0, 0, ""), (k, s, missing, not_once, bad)
+
+
+def test_failed_batch_plan_does_not_stay(host):
+    """The same for a batch, whose graph refers to the plan's buffers."""
+    r = host("""
+    from dalton_b200.batch import BatchBuilder
+    fbs = [builder("cc-pVDZ", n) for n in (1, 2)]
+    bb = BatchBuilder(fbs)
+    buf = np.zeros(2 * bb.total)
+
+    def build(t):
+        opt = _lib.default_options(thrs=t)
+        p = buf.ctypes.data
+        return _lib.load().dgf_fock_batch(bb._h, p, p + 8 * bb.total, ctypes.byref(opt), 1, None, None)
+
+    a, b = 1e-2, 1e-7
+    F.fake_reset()
+    assert build(a) == 0
+    n = F.fake_quartets()
+    calls = F.fake_malloc_calls()
+    assert build(b) == 0
+    calls = F.fake_malloc_calls() - calls
+    res = []
+    for k in range(calls):
+        assert build(a) == 0
+        F.fake_fail_malloc(k, 1)
+        s = build(b)
+        F.fake_fail_malloc(0, 0)
+        for _ in range(2):
+            F.fake_reset()
+            r = build(a)
+            res.append([s, r, F.fake_quartets() - n, F.fake_not_once(), F.fake_bad().decode()])
+    out(res=res)
+    """)
+    assert len(r["res"]) >= 6 and all(x == [2, 0, 0, 0, ""] for x in r["res"]), r["res"]
