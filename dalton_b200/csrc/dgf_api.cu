@@ -646,6 +646,15 @@ static int build_working_basis(dgf_ctx *c, const dgf_basis *b) {
   return DGF_OK;
 }
 
+static void set_default_tuning(dgf_ctx *c) {
+  for (int X = 0; X < kNumPairClass; ++X)
+    for (int Y = 0; Y < kNumPairClass; ++Y) {
+      c->split_ok[X][Y] = 1;
+      c->choice[X][Y][0] = c->choice[X][Y][1] = kDefaultVariant;
+    }
+  ++c->gen;
+}
+
 static int upload_working_maps(dgf_ctx *c) {
   const WorkMapHost &wm = c->wmap;
   std::vector<int> ints;
@@ -674,11 +683,7 @@ static int upload_working_maps(dgf_ctx *c) {
   }
   if (!shinfo.empty())
     DGF_CUDA_CHECK(cudaMemcpy(c->d_shinfo, shinfo.data(), shinfo.size() * sizeof(int), cudaMemcpyHostToDevice));
-  for (int X = 0; X < kNumPairClass; ++X)
-    for (int Y = 0; Y < kNumPairClass; ++Y) {
-      c->split_ok[X][Y] = 1;
-      c->choice[X][Y][0] = c->choice[X][Y][1] = kDefaultVariant;
-    }
+  set_default_tuning(c);
   return DGF_OK;
 }
 
@@ -741,6 +746,19 @@ static void keep_basis(dgf_ctx *c, const dgf_basis *b) {
 
 static int create_ctx(const dgf_basis *b, int device, bool resolve_all, dgf_ctx **out);
 
+static void set_tuning(dgf_ctx *c, const dgf_tuning &t) {
+  memcpy(c->choice, t.choice, sizeof(c->choice));
+  memcpy(c->split_ok, t.split_ok, sizeof(c->split_ok));
+  ++c->gen;
+}
+
+static dgf_tuning tuning_of(const dgf_ctx *c) {
+  dgf_tuning t;
+  memcpy(t.choice, c->choice, sizeof(t.choice));
+  memcpy(t.split_ok, c->split_ok, sizeof(t.split_ok));
+  return t;
+}
+
 int direct_ctx(dgf_ctx *c, bool sharded, dgf_ctx **out) {
   *out = c;
   if (!c->prim_fits || (!sharded && (c->user_tuned || c->prim_failed))) return DGF_OK;
@@ -752,6 +770,7 @@ int direct_ctx(dgf_ctx *c, bool sharded, dgf_ctx **out) {
       cudaGetLastError();
       return sharded ? r : DGF_OK;
     }
+    if (c->prim_tuning) set_tuning(c->prim, *c->prim_tuning);
   }
   *out = c->prim;
   return DGF_OK;
@@ -2027,10 +2046,20 @@ extern "C" const char *dgf_last_error(void) { return dgf::g_last_error.c_str(); 
 // similar molecules share a tuning run).
 extern "C" int dgf_copy_tuning(dgf_ctx *dst, const dgf_ctx *src) {
   if (!dst || !src) DGF_FAIL(DGF_ERR_ARG, "NULL context");
-  memcpy(dst->choice, src->choice, sizeof(dst->choice));
-  memcpy(dst->split_ok, src->split_ok, sizeof(dst->split_ok));
+  // what src's direct builds run with: its resolved context's choices, those
+  // waiting for it, or, of a context without one, its own
+  const bool made = src->prim != nullptr, waiting = !made && src->prim_tuning, none = !made && !src->prim_fits;
+  std::unique_ptr<dgf_tuning> direct;
+  if (made || waiting || none)
+    direct.reset(new dgf_tuning(made ? tuning_of(src->prim) : waiting ? *src->prim_tuning : tuning_of(src)));
+  set_tuning(dst, tuning_of(src));
   dst->user_tuned = src->user_tuned;
-  ++dst->gen;
+  if (!dst->prim)
+    dst->prim_tuning = std::move(direct);
+  else if (direct)
+    set_tuning(dst->prim, *direct);
+  else
+    set_default_tuning(dst->prim);
   return DGF_OK;
 }
 
@@ -2054,16 +2083,11 @@ extern "C" int dgf_set_class_kernel(dgf_ctx *c, int la, int lb, int lc, int ld, 
 }
 
 // Per-class autotuner: times every candidate kernel of every class pair of
-// the current plan on the given density (team kernel and each thread-kernel
-// chunk variant, FP64 and FP32) with CUDA events and keeps the fastest.
-extern "C" int dgf_autotune(dgf_ctx *c, const double *dmat_device, const dgf_options *opt, void *stream,
-                            char *report, size_t report_len) {
-  if (!c || !dmat_device) DGF_FAIL(DGF_ERR_ARG, "NULL argument");
-  DeviceGuard g(c->device);
-  dgf_options o;
-  dgf_default_options(&o);
-  if (opt) o = *opt;
-  cudaStream_t st = (cudaStream_t)stream;
+// the current plan on the given density (row, pack, warp and team kernels and
+// each thread-kernel chunk variant, FP64 and FP32) with CUDA events and keeps
+// the fastest.
+static int autotune_ctx(dgf_ctx *c, const double *dmat_device, const dgf_options &o, cudaStream_t st,
+                        std::string &rep) {
   int r = build_plan(c, o.thrs);
   if (r) return r;
   r = ensure_slots(c, 1);
@@ -2078,7 +2102,7 @@ extern "C" int dgf_autotune(dgf_ctx *c, const double *dmat_device, const dgf_opt
   cudaEvent_t e0, e1;
   DGF_CUDA_CHECK(cudaEventCreate(&e0));
   DGF_CUDA_CHECK(cudaEventCreate(&e1));
-  std::string rep = "[";
+  rep = "[";
   ++c->gen;
   c->row_slot = kRowSlots;  // the first row launch clears the task counters
   const int saved_prof = c->profiling;
@@ -2227,6 +2251,33 @@ extern "C" int dgf_autotune(dgf_ctx *c, const double *dmat_device, const dgf_opt
   rep += "]";
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  return DGF_OK;
+}
+
+// A segmented basis is tuned in both forms: the resolved one, which direct
+// builds, gradients and batches run in and which the report is of, and the
+// context's own, for the store and for builds after a kernel was pinned.
+extern "C" int dgf_autotune(dgf_ctx *c, const double *dmat_device, const dgf_options *opt, void *stream,
+                            char *report, size_t report_len) {
+  if (!c || !dmat_device) DGF_FAIL(DGF_ERR_ARG, "NULL argument");
+  DeviceGuard g(c->device);
+  dgf_options o;
+  dgf_default_options(&o);
+  if (opt) o = *opt;
+  cudaStream_t st = (cudaStream_t)stream;
+  std::string rep, own;
+  int r = autotune_ctx(c, dmat_device, o, st, own);
+  if (r) return r;
+  dgf_ctx *d = nullptr;
+  if ((r = direct_ctx(c, false, &d))) return r;
+  if (d != c) {
+    dgf_options od = o;
+    od.thrs *= kPrimThrs;
+    r = autotune_ctx(d, dmat_device, od, st, rep);
+    if (r) return r;
+  } else {
+    rep.swap(own);
+  }
   if (report && report_len) {
     strncpy(report, rep.c_str(), report_len - 1);
     report[report_len - 1] = 0;

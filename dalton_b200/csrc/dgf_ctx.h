@@ -2,6 +2,8 @@
 // shell-pair data and the per-call scratch of one molecule/basis.
 #pragma once
 
+#include <memory>
+
 #include "../../include/dgfock.h"
 #include "dgf_internal.h"
 #include "dgf_work.h"
@@ -56,6 +58,12 @@ struct dgf_graph {
   int64_t seen;
 };
 
+// Kernel choices kept for a resolved context that is not made yet.
+struct dgf_tuning {
+  int choice[dgf::kNumPairClass][dgf::kNumPairClass][2];
+  int split_ok[dgf::kNumPairClass][dgf::kNumPairClass];
+};
+
 struct dgf_ctx {
   int device = 0, nbf = 0, natom = 0, nshell = 0, spherical = 1, maxl = 0, nsm = 148;
   std::vector<double> xyz, charge;
@@ -78,6 +86,7 @@ struct dgf_ctx {
   bool prim_failed = false;   // it could not be made here (no memory): this context serves the whole builds
   bool user_tuned = false;    // a kernel was pinned on this context: it serves all calls itself, shards excepted
   dgf_ctx *prim = nullptr;
+  std::unique_ptr<dgf_tuning> prim_tuning;  // copied choices `prim` starts with (null: the defaults)
   dgf_basis basis_copy = {};
   std::vector<dgf_int> basis_i;
   std::vector<double> basis_d;

@@ -279,11 +279,15 @@ int dgf_fock_batch(dgf_batch *batch, const double *dmat_packed_device, double *f
 
 /* Per-class autotuner (no counterpart in Dalton): times every candidate
  * kernel of every quartet class of the plan for opt->thrs on the density
- * dmat_device (N x N, device) -- the row kernel, the warp kernels, the
+ * dmat_device (N x N, device) -- the row, pack and warp kernels, the
  * cooperative team kernel and the thread-per-quartet kernel in its A-chunk
  * variants, FP64 and FP32 -- and
  * keeps the fastest per class and precision in the context for later builds.
- * A JSON list of the timings is written to `report` (may be NULL). */
+ * A basis with segmented contractions is tuned in both forms: the resolved
+ * one that its direct builds, gradients and batches run in, and the
+ * contracted one of the integral store and of pinned contexts.
+ * A JSON list of the timings, of the resolved form where there is one, is
+ * written to `report` (may be NULL). */
 int dgf_autotune(dgf_ctx *ctx, const double *dmat_device, const dgf_options *opt, void *stream, char *report,
                  size_t report_len);
 

@@ -95,7 +95,7 @@ def test_batch_mixed_form(cuda):
     from dalton_b200.batch import BatchBuilder
 
     fbs, ds, big = _batch(cuda, nmol=8, seed=12)
-    fbs[big].autotune(ds[big], mixed_cutoff=1e-6)
+    report = fbs[big].autotune(ds[big], mixed_cutoff=1e-6)
     ref = [fb.herfck_device(d).clone() for fb, d in zip(fbs, ds)]
     bb = BatchBuilder(fbs)
     dp = bb.pack(ds)
@@ -109,6 +109,12 @@ def test_batch_mixed_form(cuda):
         de = max(abs(0.5 * float(torch.sum(d * (a - b)))) for d, a, b in zip(ds, bb.unpack(fp), ref))
         print(f"mixed batch: max |dF| {err:.2e}, max |dE| {de:.2e}, FP32 quartets {st['quartets_fp32']}")
         assert err < 1e-6 and de < 1e-6
+        assert (st["quartets_fp32"] > 0) == any(r.get("split") for r in report)
+    # untuned, the classes without a row kernel split
+    un = BatchBuilder([FockBuilder(fb.basis) for fb in fbs])
+    fm = un.unpack(un.herfck_batch(dp, mixed_cutoff=1e-6))
+    assert un.last_stats["quartets_fp32"] > 0
+    assert max(float(torch.max(torch.abs(a - b))) for a, b in zip(fm, ref)) < 1e-6
     # the FP64 form is unchanged after mixed calls (a separate graph)
     fp = bb.herfck_batch(dp, use_graph=True)
     for a, b in zip(bb.unpack(fp), ref):

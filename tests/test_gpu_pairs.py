@@ -104,6 +104,47 @@ def test_resolved_contractions(cuda, orc, name):
     assert float((res.herfck_stored(dt) - res.herfck_device(dt)).abs().max()) < 1e-11
 
 
+# dgf_class_time.kernel of each kernel variant (thread variants: 0)
+KERNEL_OF = {-6: 10, -5: 8, -4: 6, -3: 4, -2: 2, -1: 1}
+
+
+def _kernels(fb, d, **o):
+    fb.set_profiling(True)
+    fb.herfck_device(d, **o)
+    fb.set_profiling(False)
+    return {((r["la"], r["lb"], r["lc"], r["ld"]), r["precision"]): r["kernel"] for r in fb.profile()}
+
+
+@pytest.mark.parametrize("basis", ["6-31G*", "STO-3G", "cc-pVDZ"])
+def test_autotune_reaches_the_builds(cuda, basis):
+    """A build after the autotuner runs the kernels that its report has as the
+    fastest, also where the basis is resolved, on the tuned context and on one
+    that took the tuning over before or after its own first build; the mixed
+    form splits the classes that the tuner split."""
+    import torch
+
+    bs = build_basis(molecules.water_cluster(2, seed=3), basis)
+    d = torch.tensor(_density(bs.nbf, 8), device=cuda)
+    fb, early, late = FockBuilder(bs), FockBuilder(bs), FockBuilder(bs)
+    late.herfck_device(d)
+    ref = early.herfck_device(d) if basis == "cc-pVDZ" else FockBuilder(bs).herfck_device(d)
+    report = fb.autotune(d, mixed_cutoff=1e-6)
+    for other in (early, late):
+        other.copy_tuning_from(fb)
+    best = {}
+    for r in report:
+        if r.get("precision") == 64 and r["ms"] < best.get(tuple(r["class"]), (1e30, 0))[0]:
+            best[tuple(r["class"])] = (r["ms"], r["variant"])
+    split = {tuple(r["class"]) for r in report if r.get("split")}
+    assert best
+    for b in (fb, early, late):
+        used = _kernels(b, d)
+        assert used == {(c, 64): KERNEL_OF.get(v, 0) for c, (_, v) in best.items()}
+        mixed = _kernels(b, d, mixed_cutoff=1e-6)
+        assert {c for c, p in mixed if p == 32} == split
+        assert float((b.herfck_device(d) - ref).abs().max()) < 1e-15 * bs.nbf * max(1.0, float(ref.abs().max()))
+
+
 @pytest.mark.parametrize("basis", ["6-31G*", "cc-pVDZ"])
 def test_batch_rows(cuda, basis):
     """Batched builds with the row kernels: molecules of one to five waters,
