@@ -131,15 +131,17 @@ def test_autotune_reaches_the_builds(cuda, basis):
     report = fb.autotune(d, mixed_cutoff=1e-6)
     for other in (early, late):
         other.copy_tuning_from(fb)
-    best = {}
+    ms, best = {}, {}
     for r in report:
-        if r.get("precision") == 64 and r["ms"] < best.get(tuple(r["class"]), (1e30, 0))[0]:
-            best[tuple(r["class"])] = (r["ms"], r["variant"])
+        if r.get("precision") == 64:
+            ms.setdefault(tuple(r["class"]), {})[KERNEL_OF.get(r["variant"], 0), r["variant"]] = r["ms"]
+    for c, t in ms.items():  # the report's times are rounded: kernels at the least one are all the fastest
+        best[c, 64] = {k for (k, _), x in t.items() if x == min(t.values())}
     split = {tuple(r["class"]) for r in report if r.get("split")}
     assert best
     for b in (fb, early, late):
         used = _kernels(b, d)
-        assert used == {(c, 64): KERNEL_OF.get(v, 0) for c, (_, v) in best.items()}
+        assert used.keys() == best.keys() and all(used[c] in best[c] for c in used)
         mixed = _kernels(b, d, mixed_cutoff=1e-6)
         assert {c for c, p in mixed if p == 32} == split
         assert float((b.herfck_device(d) - ref).abs().max()) < 1e-15 * bs.nbf * max(1.0, float(ref.abs().max()))
