@@ -1486,6 +1486,12 @@ static dgf_graph *graph_entry(dgf_ctx *c, const std::string &key) {
   return &c->graphs[0];
 }
 
+static bool is_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 // stored = true: the conventional form, digesting the blocks of the integral
 // store (dgf_store_integrals) instead of evaluating integrals.
 static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double *dmat_dev, double *fmat_dev,
@@ -1780,9 +1786,7 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
     // plan and the options only, not on the caller's matrices.
     dgf_graph *gr = nullptr;
     if (seconds < kGraphSeconds && !c->profiling && nslot_total <= chunk) {
-      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-      if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
-      if (cap == cudaStreamCaptureStatusNone) {
+      if (!is_capturing(st)) {
         std::string key;
         auto add = [&key](const auto &v) { key.append(reinterpret_cast<const char *>(&v), sizeof(v)); };
         add(c->gen);
@@ -1865,15 +1869,34 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
   return DGF_OK;
 }
 
+// Whether c has the plan and the buffers of a build with these options.
+static bool build_ready(const dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const dgf_options &o, double thrs) {
+  int nslot = 0;
+  for (int k = 0; k < ndmat; ++k) nslot += ifctyp[k] / 10 == 0 ? 2 : 1;
+  nslot = std::min(nslot, kMaxSlots);
+  return !c->plan.empty() && c->plan_thrs == thrs && c->cap_slots >= nslot &&
+         (o.ifthrs >= 16 || c->cap_blk_slots >= nslot);
+}
+
 // A direct build of c, in its resolved context where there is one.
 static int fock_direct(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double *dmat_dev, double *fmat_dev,
                        const dgf_options *opt, cudaStream_t st, dgf_stats *stats) {
-  dgf_ctx *d = nullptr;
-  if (const int r = direct_ctx(c, opt && opt->shard_count > 1, &d)) return r;
-  if (d == c) return fock_impl(c, ndmat, ifctyp, dmat_dev, fmat_dev, opt, st, stats);
   dgf_options o;
   dgf_default_options(&o);
   if (opt) o = *opt;
+  const bool sharded = o.shard_count > 1;
+  // Inside the caller's stream capture nothing can be made: where the resolved
+  // form is not there or not ready, this context serves with the plan that a
+  // store or a stored build made.  Not a shard, which all ranks cut alike.
+  if (c->prim_fits && !(c->prim && build_ready(c->prim, ndmat, ifctyp, o, o.thrs * kPrimThrs)) && is_capturing(st)) {
+    if (sharded)
+      DGF_FAIL(DGF_ERR_ARG, "a shard in a stream capture needs the same call once before the capture");
+    if (!c->prim || build_ready(c, ndmat, ifctyp, o, o.thrs))
+      return fock_impl(c, ndmat, ifctyp, dmat_dev, fmat_dev, opt, st, stats);
+  }
+  dgf_ctx *d = nullptr;
+  if (const int r = direct_ctx(c, sharded, &d)) return r;
+  if (d == c) return fock_impl(c, ndmat, ifctyp, dmat_dev, fmat_dev, opt, st, stats);
   o.thrs *= kPrimThrs;
   d->profiling = c->profiling;
   const int r = fock_impl(d, ndmat, ifctyp, dmat_dev, fmat_dev, &o, st, stats);

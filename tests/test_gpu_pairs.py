@@ -167,3 +167,28 @@ def test_batch_rows(cuda, basis):
                 assert float((a - b).abs().max()) < 1e-14 * a.shape[0] * max(1.0, float(b.abs().max()))
         fm = bb.unpack(bb.herfck_batch(bb.pack(ds), use_graph=False, mixed_cutoff=1e-7))
         assert max(float((a - b).abs().max()) for a, b in zip(fm, ref)) < 1e-6
+
+
+def test_capture_after_a_store(cuda):
+    """A build captured into the caller's graph when only the integral store
+    made a plan before: the contracted context serves it."""
+    import torch
+
+    bs = build_basis(molecules.water_cluster(2, seed=3), "6-31G*")
+    fb = FockBuilder(bs)
+    warm = FockBuilder(bs)
+    warm.set_class_kernel((1, 0, 0, 0), 0)
+    warm.herfck_device(torch.zeros((bs.nbf, bs.nbf), dtype=torch.float64, device=cuda))  # loads the kernels
+    fb.store_integrals()
+    d = torch.tensor(_density(bs.nbf, 1), device=cuda)
+    f = torch.empty_like(d)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        fb.herfck_device(d, fmat=f, stats=False)
+    for seed in (2, 3):
+        d.copy_(torch.tensor(_density(bs.nbf, seed), device=cuda))
+        g.replay()
+        torch.cuda.synchronize()
+        ref = FockBuilder(bs).herfck_device(d)
+        assert float((f - ref).abs().max()) < 1e-11 * max(1.0, float(ref.abs().max()))

@@ -209,3 +209,40 @@ def test_failed_batch_plan_does_not_stay(host):
     out(res=res)
     """)
     assert len(r["res"]) >= 6 and all(x == [2, 0, 0, 0, ""] for x in r["res"]), r["res"]
+
+
+@pytest.mark.parametrize("basis", ["6-31G*", "cc-pVDZ"])
+def test_capture_after_a_store(host, basis):
+    """Inside the caller's stream capture, where nothing can be allocated, a
+    direct build runs on the plan that a store made, as every context does
+    whose own direct builds use that plan; a shard, which must not, says what
+    it needs."""
+    r = host(f"""
+    fb, other = builder({basis!r}), builder({basis!r})
+    lib = _lib.load()
+    t = 1e-6
+    assert lib.dgf_store_integrals(fb._h, t, 0, None, None) == 0
+    buf = np.zeros((2, fb.nbf, fb.nbf))
+    ift = (_lib.dgf_int * 1)(13)
+
+    def build(b, n=1, **o):
+        opt = _lib.default_options(thrs=t, shard_count=n, **o)
+        F.fake_reset()
+        s = lib.dgf_fock_device(b._h, 1, ift, buf[0].ctypes.data, buf[1].ctypes.data, ctypes.byref(opt), None, None)
+        return [s, F.fake_quartets(), F.fake_not_once(), F.fake_bad().decode()]
+
+    F.fake_user_capture(1)
+    captured, shard, screened = build(fb), build(fb, 2), build(fb, ifthrs=10)
+    F.fake_user_capture(0)
+    other.set_class_kernel((1, 0, 0, 0), 0)  # serves its whole builds itself
+    own = build(other)
+    after = [build(fb), build(fb, 2)]
+    F.fake_user_capture(1)
+    again = [build(fb), build(fb, 2)]
+    out(captured=captured, shard=shard, screened=screened, own=own, after=after, again=again)
+    """)
+    assert r["captured"] == r["own"] and r["own"][0] == 0 and r["own"][3] == ""
+    assert r["shard"][0] == (1 if basis == "6-31G*" else 0)
+    assert r["screened"][0] != 0  # its buffers were not there: an error, not a crash
+    assert [x[0] for x in r["after"] + r["again"]] == [0] * 4
+    assert r["after"] == r["again"]
