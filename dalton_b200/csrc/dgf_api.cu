@@ -1822,10 +1822,17 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
       if (!r && e == cudaSuccess) e = cudaGraphInstantiate(&gr->exec, g, 0);
       if (g) cudaGraphDestroy(g);
       if (r) return r;
-      if (e != cudaSuccess) gr->exec = nullptr;
-      DGF_CUDA_CHECK(e);
       gr->launches = launches - l0;
-      DGF_CUDA_CHECK(cudaGraphLaunch(gr->exec, st));
+      if (e == cudaSuccess) {
+        DGF_CUDA_CHECK(cudaGraphLaunch(gr->exec, st));
+      } else {  // no graph (no memory for it): launched as the first call, and tried again two calls on
+        cudaGetLastError();
+        gr->exec = nullptr;
+        gr->seen = 0;
+        launches = l0;
+        r = enqueue_all(st);
+        if (r) return r;
+      }
     } else {
       r = enqueue_all(st);
       if (r) return r;

@@ -246,3 +246,25 @@ def test_capture_after_a_store(host, basis):
     assert r["screened"][0] != 0  # its buffers were not there: an error, not a crash
     assert [x[0] for x in r["after"] + r["again"]] == [0] * 4
     assert r["after"] == r["again"]
+
+
+def test_build_without_a_graph(host):
+    """A short build whose graph cannot be made is launched without one, and
+    replayed as a graph once it can be."""
+    r = host("""
+    fb = builder("cc-pVDZ")
+    d = eye(fb)
+    F.fake_fail_instantiate(2)
+    res = []
+    for _ in range(8):
+        replays = F.fake_replays()
+        F.fake_reset()
+        s = status(fb.herfck, d, thrs=1e-6)
+        res.append([s, F.fake_quartets(), F.fake_not_once(), F.fake_bad().decode(), F.fake_replays() - replays,
+                    fb.last_stats["kernel_launches"]])
+    out(res=res)
+    """)
+    assert r["res"][0][1] > 0
+    for x in r["res"]:
+        assert x[:4] == [0, r["res"][0][1], 0, ""] and x[5] == r["res"][0][5], r["res"]
+    assert [x[4] for x in r["res"]] == [0, 0, 0, 0, 0, 1, 1, 1]
