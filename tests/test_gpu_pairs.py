@@ -55,6 +55,28 @@ def test_one_electron(cuda, orc, name):
         assert np.abs(g - ref).max() < 1e-14 * bs.nbf * max(1.0, np.abs(ref).max())
 
 
+@pytest.mark.parametrize("sph", [True, False])
+def test_one_electron_of_distant_shells(cuda, orc, sph):
+    """Two atoms 10.3 bohr apart: the overlap distributions of their f shells
+    have mu R^2 just above 40, beyond the two-electron pair lists, but their
+    polynomials keep the integrals far above the block's rounding."""
+    bs = build_basis(Molecule.from_bohr(["C", "C"], [[0.1, -0.2, 0.3], [10.36, 0.3, 0.8]]), "cc-pVTZ", spherical=sph)
+    fb = FockBuilder(bs)
+    n1 = bs.nbf // 2
+    d, w = _density(bs.nbf, 1), _density(bs.nbf, 2)
+    for _ in range(2):
+        for x, y in zip(fb.oneint(), orc.oneint(bs)):
+            # the block of the two atoms by itself: elements up to 0.05
+            assert np.abs(x[:n1, n1:] - y[:n1, n1:]).max() < 1e-15
+            assert np.abs(x - y).max() < 1e-13 * max(1.0, np.abs(y).max())
+        # only the densities that couple the two atoms: the forces of far pairs alone
+        dd, ww = d.copy(), w.copy()
+        for m in (dd, ww):
+            m[:n1, :n1] = m[n1:, n1:] = 0.0
+        g, ref = fb.grad1e(dd, ww), orc.grad1e(bs, dd, ww)
+        assert np.abs(g - ref).max() < 1e-14
+
+
 @pytest.mark.parametrize("name", [n for n in MOLS if not n.startswith("ch4")])
 @pytest.mark.parametrize("hfx", [1.0, 0.0, 0.3])
 def test_bilinear_gradient(cuda, orc, name, hfx):
