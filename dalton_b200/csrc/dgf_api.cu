@@ -179,7 +179,7 @@ static void free_ctx(dgf_ctx *c) {
                   c->d_dmax,  c->d_cnt,    c->d_qoff,   c->d_wmap_i, c->d_wmap_c, c->d_wmeta, c->d_wdims, c->d_gw,
                   c->d_shinfo, c->d_blk_gab, c->d_blk_info, c->d_blk_dmax, c->d_ks_i, c->d_ks_q, c->d_ks_pp,
                   c->d_store, c->d_fine,   c->d_row_bra, c->d_row_tasks, c->d_row_work,
-                  c->d_one,   c->d_pg,    c->d_far,   c->d_far_pp};
+                  c->d_one,   c->d_pg,    c->d_one_pairs, c->d_one_pp};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (double *p : c->d_frag)
@@ -484,11 +484,10 @@ struct ShellList {
 };
 
 // Shell pairs A >= B (the higher l first) with their primitive pairs, class
-// by class, of the primitive pairs with near < mu |AB|^2 <= far.  The
+// by class; primitive pairs with mu |AB|^2 > reach are dropped.  The
 // two-electron lists stop at 40 (e^-40 ~ 4e-18).
-constexpr double kPairReach = 40.0;
 static void build_pairs(const dgf_ctx *c, const ShellList &sh, int nbfm, std::vector<PairRec> &pairs,
-                        int *cls_off, std::vector<PrimPair> &pp, double near = -1.0, double far = kPairReach) {
+                        int *cls_off, std::vector<PrimPair> &pp, double reach = 40.0) {
   const double r2pi52 = std::sqrt(2.0 * std::pow(3.14159265358979323846, 2.5));
   std::vector<std::vector<PairRec>> bycls(kNumPairClass);
   pp.clear();
@@ -520,7 +519,7 @@ static void build_pairs(const dgf_ctx *c, const ShellList &sh, int nbfm, std::ve
         for (int j = 0; j < sh.nprim[sb]; ++j) {
           const double ea = sh.a[sh.p0[sa] + i], eb = sh.a[sh.p0[sb] + j];
           const double p = ea + eb, mu = ea * eb / p;
-          if (mu * ab2 > far || !(mu * ab2 > near)) continue;
+          if (mu * ab2 > reach) continue;
           PrimPair q;
           q.p = p;
           q.Px = (ea * xa[0] + eb * xb[0]) / p;
@@ -547,29 +546,32 @@ static void build_pairs(const dgf_ctx *c, const ShellList &sh, int nbfm, std::ve
   }
 }
 
-// The primitive pairs that the two-electron lists leave out and one-electron
-// integrals need.  With x = mu |AB|^2 a pair of normalised primitives has
-// |S| <= (4 x)^{(la + lb)/2} e^-x, T and the derivatives further powers of x:
-// above 1e-12 with f shells at x = 40 (two carbon atoms in cc-pVTZ, Cartesian:
-// S 2e-12, T 4e-11, gradient 5e-12), below 1e-22 at x = 80.
-constexpr double kFarReach = 80.0;
-int far_pairs(dgf_ctx *c) {
-  if (c->far_made) return DGF_OK;
+// The pair list of the one-electron calls: all primitive pairs up to
+// x = mu |AB|^2 = 80, where the two-electron lists stop at 40.  A pair of
+// normalised primitives has |S| <= (4 x)^{(la + lb)/2} e^-x, T and the
+// derivatives further powers of x: above 1e-12 with f shells at x = 40 (two
+// carbon atoms in cc-pVTZ, Cartesian: S 2e-12, T 4e-11, gradient 5e-12),
+// below 1e-22 at x = 80.  Pairs with most primitives first, so that a warp's
+// lanes have about as many each.
+constexpr double kOneReach = 80.0;
+int one_pairs(dgf_ctx *c) {
+  if (c->one_made) return DGF_OK;
   std::vector<PairRec> pairs;
   std::vector<PrimPair> pp;
   build_pairs(c, ShellList{c->ws_l, c->ws_atom, c->ws_ao, c->ws_nprim, c->ws_p0, c->ws_a, c->ws_c, &c->ws_blk_flag},
-              c->nwf, pairs, c->far_off, pp, kPairReach, kFarReach);
-  if (!c->d_far && dev_alloc(&c->d_far, pairs.size()) != cudaSuccess) c->d_far = nullptr;
-  if (!c->d_far_pp && dev_alloc(&c->d_far_pp, pp.size()) != cudaSuccess) c->d_far_pp = nullptr;
-  if (!c->d_far || !c->d_far_pp) {
+              c->nwf, pairs, c->one_off, pp, kOneReach);
+  for (int X = 0; X < kNumPairClass; ++X)
+    std::stable_sort(pairs.begin() + c->one_off[X], pairs.begin() + c->one_off[X + 1],
+                     [](const PairRec &u, const PairRec &v) { return u.npp > v.npp; });
+  if (!c->d_one_pairs && dev_alloc(&c->d_one_pairs, pairs.size()) != cudaSuccess) c->d_one_pairs = nullptr;
+  if (!c->d_one_pp && dev_alloc(&c->d_one_pp, pp.size()) != cudaSuccess) c->d_one_pp = nullptr;
+  if (!c->d_one_pairs || !c->d_one_pp) {
     cudaGetLastError();
     DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the one-electron pairs failed");
   }
-  if (!pairs.empty()) {
-    DGF_CUDA_CHECK(cudaMemcpy(c->d_far, pairs.data(), pairs.size() * sizeof(PairRec), cudaMemcpyHostToDevice));
-    DGF_CUDA_CHECK(cudaMemcpy(c->d_far_pp, pp.data(), pp.size() * sizeof(PrimPair), cudaMemcpyHostToDevice));
-  }
-  c->far_made = true;
+  DGF_CUDA_CHECK(cudaMemcpy(c->d_one_pairs, pairs.data(), pairs.size() * sizeof(PairRec), cudaMemcpyHostToDevice));
+  DGF_CUDA_CHECK(cudaMemcpy(c->d_one_pp, pp.data(), pp.size() * sizeof(PrimPair), cudaMemcpyHostToDevice));
+  c->one_made = true;
   return DGF_OK;
 }
 

@@ -99,11 +99,11 @@ struct dgf_ctx {
   int64_t *d_wmeta = nullptr;   // {0, nwf^2} {0, nbf^2} element offsets of the single-molecule form
   int *d_wdims = nullptr;       // {nwf, nbf, 0, 0}
   double *d_one = nullptr;      // scratch of the one-electron calls (dgf_grad.cu), made by the first of them
-  // their primitive pairs beyond the two-electron lists (far_pairs), by class
-  bool far_made = false;
-  int far_off[dgf::kNumPairClass + 1] = {0};
-  dgf::PairRec *d_far = nullptr;
-  dgf::PrimPair *d_far_pp = nullptr;
+  // their pairs, by class (one_pairs)
+  bool one_made = false;
+  int one_off[dgf::kNumPairClass + 1] = {0};
+  dgf::PairRec *d_one_pairs = nullptr;
+  dgf::PrimPair *d_one_pp = nullptr;
   double *d_pg = nullptr;       // two-electron gradient: derivatives per pair (6 each), then task counters
   double *d_gw = nullptr;       // working-basis densities of the two-electron gradient (2 nwf^2)
   int *d_shinfo = nullptr;      // per working shell: first function | function count (density bounds)
@@ -193,8 +193,8 @@ struct RowSource {
   const int64_t *qoff;
   int bra0, ket0, ket_end;
 };
-// Makes the far pairs of a context (dgf_api.cu).
-int far_pairs(dgf_ctx *c);
+// Makes the pair list of a context's one-electron calls (dgf_api.cu).
+int one_pairs(dgf_ctx *c);
 
 // Appends the row tasks of a launch (dgf_api.cu).
 void row_tasks(const std::vector<RowSource> &src, int max_bras, int min_width, std::vector<int4> &tasks);

@@ -3,21 +3,20 @@
 // (HER1INT, DALTON/abacus/her1drv.F; the operators' derivative integrals,
 // DALTON/abacus/aba1mat.F).
 //
-// Both work on the shell pairs of the two-electron working basis and on the
-// primitive pairs that its screening at mu R^2 = 40 leaves out (far_pairs), class by
-// class with compile-time angular momenta: one thread per pair, everything in
-// registers for s, p and d shells, so that no index arithmetic or local
-// memory stands between the Boys functions.  A general contraction's
-// primitives are evaluated once and mapped to the AO basis afterwards
-// (S = C^T S_w C; D_w = C D C^T).  The nuclear attraction sums R_tuv over the
-// nuclei before it is contracted with the Hermite coefficients; its gradient
-// contracts the density with the differentiated coefficients first, so that a
-// nucleus costs one R_tuv and three short dot products, and the force on it
-// is summed over the warp before it is added.  Bound by FP64 arithmetic and
-// the latency of the Boys function.  Measured on (H2O)16 / cc-pVDZ (384
-// functions, 48 nuclei), both calls with their host copies: 76.4 ms with one
-// thread per ordered pair of contracted shells and run-time angular momenta,
-// 2.5 ms so.
+// Both work on the shell pairs of the two-electron working basis, in a list of
+// their own that reaches further (one_pairs), class by class with compile-time
+// angular momenta: one thread per pair, everything in registers for s, p and d
+// shells, so that no index arithmetic or local memory stands between the Boys
+// functions.  A general contraction's primitives are evaluated once and mapped
+// to the AO basis afterwards (S = C^T S_w C; D_w = C D C^T).  The nuclear
+// attraction sums R_tuv over the nuclei before it is contracted with the
+// Hermite coefficients; its gradient contracts the density with the
+// differentiated coefficients first, so that a nucleus costs one R_tuv and
+// three short dot products, and the force on it is summed over the warp before
+// it is added.  Bound by FP64 arithmetic and the latency of the Boys function.
+// Measured on (H2O)16 / cc-pVDZ (384 functions, 48 nuclei), both calls with
+// their host copies: 76.4 ms with one thread per ordered pair of contracted
+// shells and run-time angular momenta, 2.6 ms so.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -168,8 +167,7 @@ __global__ void __launch_bounds__(kOneBlock) oneint_kernel(const OneArgs a) {
           });
       }
     }
-    // half matrices: the epilogue adds the transpose.  A pair is in a list
-    // once, and the lists of a class run one after the other.
+    // half matrices: the epilogue adds the transpose
     const double w = pr.same ? 0.5 : 1.0;
     auto put = [&](double *M, const double *c) {
       if (!M) return;
@@ -181,7 +179,7 @@ __global__ void __launch_bounds__(kOneBlock) oneint_kernel(const OneArgs a) {
         for (int k = 0; k < FA * FB; ++k) f[k] = c[k];
       }
 #pragma unroll
-      for (int k = 0; k < FA * FB; ++k) M[(size_t)(pr.aoA + k / FB) * a.nwf + pr.aoB + k % FB] += w * f[k];
+      for (int k = 0; k < FA * FB; ++k) M[(size_t)(pr.aoA + k / FB) * a.nwf + pr.aoB + k % FB] = w * f[k];
     };
     put(a.S, S);
     put(a.T, T);
@@ -430,26 +428,12 @@ struct OneScratch {
 OneArgs one_args(const dgf_ctx *c, const OneScratch &s) {
   OneArgs a;
   memset(&a, 0, sizeof(a));
+  a.pp = c->d_one_pp;
   a.xyz = s.xyz;
   a.charge = s.charge;
   a.natom = c->natom;
   a.nwf = c->nwf;
   return a;
-}
-
-// f(class) with the pairs of a class in `a`: the two-electron list, then the
-// primitive pairs that it leaves out.
-template <typename F>
-void for_pair_lists(const dgf_ctx *c, OneArgs &a, F &&f) {
-  for (int X = 0; X < kNumPairClass; ++X)
-    for (int far = 0; far < 2; ++far) {
-      const int *off = far ? c->far_off : c->cls_off;
-      a.npair = off[X + 1] - off[X];
-      if (!a.npair) continue;
-      a.pairs = (far ? c->d_far : c->d_pairs) + off[X];
-      a.pp = far ? c->d_far_pp : c->d_pp;
-      f(X);
-    }
 }
 
 }  // namespace
@@ -462,19 +446,21 @@ extern "C" int dgf_oneint(dgf_ctx *c, double *S, double *T, double *V) {
   DeviceGuard g(c->device);
   OneScratch s(c);
   int r = s.open();
-  if (!r) r = far_pairs(c);
+  if (!r) r = one_pairs(c);
   if (r) return r;
   OneArgs a = one_args(c, s);
   a.S = S ? s.w : nullptr;
   a.T = T ? s.w + s.n2w : nullptr;
   a.V = V ? s.w + 2 * s.n2w : nullptr;
   cudaError_t e = cudaMemsetAsync(s.w, 0, 3 * s.n2w * 8);
-  for_pair_lists(c, a, [&](int X) {
-    if (e != cudaSuccess) return;
+  for (int X = 0; X < kNumPairClass && e == cudaSuccess; ++X) {
+    a.npair = c->one_off[X + 1] - c->one_off[X];
+    if (!a.npair) continue;
+    a.pairs = c->d_one_pairs + c->one_off[X];
     a.boys = c->d_boys + (size_t)kPairClassL[X] * kBoysTableDoubles;
     kOneint[X](a, c->spherical != 0, c->nsm);
     e = cudaGetLastError();
-  });
+  }
   double *outs[3] = {S, T, V};
   const WorkMaps maps = ctx_maps(c);
   for (int k = 0; k < 3; ++k)
@@ -498,7 +484,7 @@ extern "C" int dgf_grad1e(dgf_ctx *c, const double *dmat, const double *wmat, do
   DeviceGuard g(c->device);
   OneScratch s(c);
   int r = s.open();
-  if (!r) r = far_pairs(c);
+  if (!r) r = one_pairs(c);
   if (r) return r;
   OneArgs a = one_args(c, s);
   cudaError_t e = cudaMemcpy(s.ao, dmat, s.n2 * 8, cudaMemcpyHostToDevice);
@@ -512,12 +498,14 @@ extern "C" int dgf_grad1e(dgf_ctx *c, const double *dmat, const double *wmat, do
   a.grad = s.grad;
   a.smem_acc = c->natom <= kOneSmemAtoms;
   if (e == cudaSuccess) e = cudaGetLastError();
-  for_pair_lists(c, a, [&](int X) {
-    if (e != cudaSuccess) return;
+  for (int X = 0; X < kNumPairClass && e == cudaSuccess; ++X) {
+    a.npair = c->one_off[X + 1] - c->one_off[X];
+    if (!a.npair) continue;
+    a.pairs = c->d_one_pairs + c->one_off[X];
     a.boys = c->d_boys + (size_t)(kPairClassL[X] + 1) * kBoysTableDoubles;
     kGrad1e[X](a, c->spherical != 0, c->nsm);
     e = cudaGetLastError();
-  });
+  }
   std::vector<double> gr(3 * (size_t)c->natom);
   if (e == cudaSuccess) e = cudaMemcpy(gr.data(), s.grad, gr.size() * 8, cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) {
