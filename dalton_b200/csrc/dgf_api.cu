@@ -569,8 +569,8 @@ int one_pairs(dgf_ctx *c) {
     cudaGetLastError();
     DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the one-electron pairs failed");
   }
-  DGF_CUDA_CHECK(cudaMemcpy(c->d_one_pairs, pairs.data(), pairs.size() * sizeof(PairRec), cudaMemcpyHostToDevice));
-  DGF_CUDA_CHECK(cudaMemcpy(c->d_one_pp, pp.data(), pp.size() * sizeof(PrimPair), cudaMemcpyHostToDevice));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_one_pairs, pairs.data(), pairs.size() * sizeof(PairRec)));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_one_pp, pp.data(), pp.size() * sizeof(PrimPair)));
   c->one_made = true;
   return DGF_OK;
 }
@@ -701,10 +701,10 @@ static int upload_working_maps(dgf_ctx *c) {
     cudaGetLastError();
     DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the working-basis maps failed");
   }
-  DGF_CUDA_CHECK(cudaMemcpy(c->d_wmap_i, ints.data(), ints.size() * sizeof(int), cudaMemcpyHostToDevice));
-  if (!cs.empty()) DGF_CUDA_CHECK(cudaMemcpy(c->d_wmap_c, cs.data(), cs.size() * 8, cudaMemcpyHostToDevice));
-  DGF_CUDA_CHECK(cudaMemcpy(c->d_wmeta, meta, sizeof(meta), cudaMemcpyHostToDevice));
-  DGF_CUDA_CHECK(cudaMemcpy(c->d_wdims, dims, sizeof(dims), cudaMemcpyHostToDevice));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_wmap_i, ints.data(), ints.size() * sizeof(int)));
+  if (!cs.empty()) DGF_CUDA_CHECK(upload(c->stream, c->d_wmap_c, cs.data(), cs.size() * 8));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_wmeta, meta, sizeof(meta)));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_wdims, dims, sizeof(dims)));
   std::vector<int> shinfo(c->ws_ao);
   for (int s = 0; s < c->nwshell; ++s) shinfo.push_back(nfun(c->ws_l[s], c->spherical));
   if (dev_alloc(&c->d_shinfo, std::max<size_t>(shinfo.size(), 1)) != cudaSuccess) {
@@ -712,7 +712,7 @@ static int upload_working_maps(dgf_ctx *c) {
     DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the shell table failed");
   }
   if (!shinfo.empty())
-    DGF_CUDA_CHECK(cudaMemcpy(c->d_shinfo, shinfo.data(), shinfo.size() * sizeof(int), cudaMemcpyHostToDevice));
+    DGF_CUDA_CHECK(upload(c->stream, c->d_shinfo, shinfo.data(), shinfo.size() * sizeof(int)));
   set_default_tuning(c);
   return DGF_OK;
 }
@@ -914,12 +914,12 @@ static int create_ctx(const dgf_basis *b, int device, bool resolve_all, dgf_ctx 
     cudaGetLastError();
     DGF_FAIL(DGF_ERR_NOMEM, "device allocation failed while creating the context");
   }
-  DGF_CUDA_CHECK(cudaMemcpy(c->d_boys, boys.data(), boys.size() * 8, cudaMemcpyHostToDevice));
-  DGF_CUDA_CHECK(cudaMemcpy(c->d_sph, sph.data(), sph.size() * 8, cudaMemcpyHostToDevice));
-  DGF_CUDA_CHECK(cudaMemcpy(c->d_fine, fine.data(), fine.size() * 8, cudaMemcpyHostToDevice));
-  DGF_CUDA_CHECK(cudaMemcpy(c->d_pp, c->pp.data(), c->pp.size() * sizeof(PrimPair), cudaMemcpyHostToDevice));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_boys, boys.data(), boys.size() * 8));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_sph, sph.data(), sph.size() * 8));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_fine, fine.data(), fine.size() * 8));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_pp, c->pp.data(), c->pp.size() * sizeof(PrimPair)));
   DGF_CUDA_CHECK(
-      cudaMemcpy(c->d_pairs, c->pairs.data(), c->pairs.size() * sizeof(PairRec), cudaMemcpyHostToDevice));
+      upload(c->stream, c->d_pairs, c->pairs.data(), c->pairs.size() * sizeof(PairRec)));
   int st = upload_working_maps(c.get());
   if (st) return st;
   st = compute_schwarz(c.get());
@@ -960,9 +960,9 @@ static int create_ctx(const dgf_basis *b, int device, bool resolve_all, dgf_ctx 
     }
     c->pp.swap(pp2);
   }
-  DGF_CUDA_CHECK(cudaMemcpy(c->d_pp, c->pp.data(), c->pp.size() * sizeof(PrimPair), cudaMemcpyHostToDevice));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_pp, c->pp.data(), c->pp.size() * sizeof(PrimPair)));
   DGF_CUDA_CHECK(
-      cudaMemcpy(c->d_pairs, c->pairs.data(), c->pairs.size() * sizeof(PairRec), cudaMemcpyHostToDevice));
+      upload(c->stream, c->d_pairs, c->pairs.data(), c->pairs.size() * sizeof(PairRec)));
   // Bra pairs of every class in row order.
   c->row_bra.resize(c->pairs.size());
   for (int X = 0; X < kNumPairClass; ++X) {
@@ -978,7 +978,7 @@ static int create_ctx(const dgf_basis *b, int device, bool resolve_all, dgf_ctx 
     });
   }
   if (!c->row_bra.empty())
-    DGF_CUDA_CHECK(cudaMemcpy(c->d_row_bra, c->row_bra.data(), c->row_bra.size() * sizeof(int), cudaMemcpyHostToDevice));
+    DGF_CUDA_CHECK(upload(c->stream, c->d_row_bra, c->row_bra.data(), c->row_bra.size() * sizeof(int)));
   // Ket table of single-primitive kets (first primitive pair of every pair).
   if (c->nwshell < 65536 && !c->pairs.empty()) {
     const size_t np = c->pairs.size();
@@ -997,9 +997,9 @@ static int create_ctx(const dgf_basis *b, int device, bool resolve_all, dgf_ctx 
       cudaGetLastError();
       DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the ket table failed");
     }
-    DGF_CUDA_CHECK(cudaMemcpy(c->d_ks_i, ki.data(), np * sizeof(int4), cudaMemcpyHostToDevice));
-    DGF_CUDA_CHECK(cudaMemcpy(c->d_ks_q, kq.data(), np * 8, cudaMemcpyHostToDevice));
-    DGF_CUDA_CHECK(cudaMemcpy(c->d_ks_pp, kp.data(), 11 * np * 8, cudaMemcpyHostToDevice));
+    DGF_CUDA_CHECK(upload(c->stream, c->d_ks_i, ki.data(), np * sizeof(int4)));
+    DGF_CUDA_CHECK(upload(c->stream, c->d_ks_q, kq.data(), np * 8));
+    DGF_CUDA_CHECK(upload(c->stream, c->d_ks_pp, kp.data(), 11 * np * 8));
   }
   *out = c.release();
   return DGF_OK;
@@ -1037,8 +1037,8 @@ extern "C" int dgf_count_ao_quartets(dgf_ctx *c, double thrs, dgf_int *count) {
     if (d_pairs) cudaFree(d_pairs);
     DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the AO pair list failed");
   }
-  cudaError_t e = cudaMemcpy(d_pairs, pairs.data(), pairs.size() * sizeof(PairRec), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(d_pp, pp.data(), pp.size() * sizeof(PrimPair), cudaMemcpyHostToDevice);
+  cudaError_t e = upload(c->stream, d_pairs, pairs.data(), pairs.size() * sizeof(PairRec));
+  if (e == cudaSuccess) e = upload(c->stream, d_pp, pp.data(), pp.size() * sizeof(PrimPair));
   std::vector<double> q;
   int st = (e == cudaSuccess) ? schwarz_of(c, d_pairs, d_pp, cls_off, q) : DGF_ERR_CUDA;
   cudaFree(d_pairs);
@@ -1251,7 +1251,10 @@ static int build_plan(dgf_ctx *c, double thrs) {
         }
       }
     }
-  c->plan.clear();  // its buffers are replaced below: a failure on the way leaves no plan
+  // its buffers are replaced below: a failure on the way leaves no plan, and
+  // builds on any stream that still read them end first
+  c->plan.clear();
+  if (c->d_qoff) DGF_CUDA_CHECK(cudaDeviceSynchronize());
   if (tasks.size() > c->row_tasks_cap) {
     if (c->d_row_tasks) cudaFree(c->d_row_tasks);
     c->d_row_tasks = nullptr;
@@ -1263,7 +1266,7 @@ static int build_plan(dgf_ctx *c, double thrs) {
     c->row_tasks_cap = tasks.size();
   }
   if (!tasks.empty())
-    DGF_CUDA_CHECK(cudaMemcpy(c->d_row_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    DGF_CUDA_CHECK(upload(c->stream, c->d_row_tasks, tasks.data(), tasks.size() * sizeof(int4)));
   if (all.size() > c->qoff_cap) {
     if (c->d_qoff) cudaFree(c->d_qoff);
     c->d_qoff = nullptr;
@@ -1274,7 +1277,7 @@ static int build_plan(dgf_ctx *c, double thrs) {
     }
     c->qoff_cap = all.size();
   }
-  DGF_CUDA_CHECK(cudaMemcpy(c->d_qoff, all.data(), all.size() * 8, cudaMemcpyHostToDevice));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_qoff, all.data(), all.size() * 8));
   if (const int r = ensure_frags(c, plan)) return r;
   c->plan.swap(plan);
   c->plan_thrs = thrs;
@@ -1384,8 +1387,8 @@ static int ensure_block_screen(dgf_ctx *c, int nslot) {
       if (d_pairs) cudaFree(d_pairs);
       DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the AO pair list failed");
     }
-    cudaError_t e = cudaMemcpy(d_pairs, pairs.data(), pairs.size() * sizeof(PairRec), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(d_pp, pp.data(), pp.size() * sizeof(PrimPair), cudaMemcpyHostToDevice);
+    cudaError_t e = upload(c->stream, d_pairs, pairs.data(), pairs.size() * sizeof(PairRec));
+    if (e == cudaSuccess) e = upload(c->stream, d_pp, pp.data(), pp.size() * sizeof(PrimPair));
     std::vector<double> q;
     int st = (e == cudaSuccess) ? schwarz_of(c, d_pairs, d_pp, cls_off, q) : DGF_ERR_CUDA;
     cudaFree(d_pairs);
@@ -1404,8 +1407,8 @@ static int ensure_block_screen(dgf_ctx *c, int nslot) {
       cudaGetLastError();
       DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the block Schwarz factors failed");
     }
-    DGF_CUDA_CHECK(cudaMemcpy(c->d_blk_gab, gab.data(), nb2 * 8, cudaMemcpyHostToDevice));
-    DGF_CUDA_CHECK(cudaMemcpy(c->d_blk_info, info.data(), info.size() * sizeof(int), cudaMemcpyHostToDevice));
+    DGF_CUDA_CHECK(upload(c->stream, c->d_blk_gab, gab.data(), nb2 * 8));
+    DGF_CUDA_CHECK(upload(c->stream, c->d_blk_info, info.data(), info.size() * sizeof(int)));
   }
   if (nslot > c->cap_blk_slots) {
     ++c->gen;

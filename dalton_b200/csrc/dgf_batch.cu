@@ -299,23 +299,23 @@ extern "C" int dgf_batch_create(dgf_ctx *const *caller_ctxs, dgf_int nmol, dgf_b
     batch_free(b);
     BFAIL(DGF_ERR_NOMEM, "device allocation for the batch failed");
   }
-  e = cudaMemcpy(b->d_pairs, b->pairs.data(), b->pairs.size() * sizeof(PairRec), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_pp, pp.data(), pp.size() * sizeof(PrimPair), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_boys, ctxs[0]->d_boys, n_boys * 8, cudaMemcpyDeviceToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_sph, ctxs[0]->d_sph, kSphTableDoubles * 8, cudaMemcpyDeviceToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_offsets, offs.data(), offs.size() * 8, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_dims, dims.data(), dims.size() * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_wmap_i, ints.data(), ints.size() * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !cs.empty()) e = cudaMemcpy(b->d_wmap_c, cs.data(), cs.size() * 8, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && npair) e = cudaMemcpy(b->d_row_bra, b->row_bra.data(), npair * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && npair) e = cudaMemcpy(b->d_ks_i, ki.data(), npair * sizeof(int4), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && npair) e = cudaMemcpy(b->d_ks_q, kq.data(), npair * 8, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && npair) e = cudaMemcpy(b->d_ks_pp, kp.data(), 11 * npair * 8, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_fine, ctxs[0]->d_fine, n_fine * 8, cudaMemcpyDeviceToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_bsh, bsh.data(), bsh.size() * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_bmol, bmol.data(), bmol.size() * 4, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_bpref, bpref.data(), bpref.size() * 8, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
+  e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = upload(b->stream, b->d_pairs, b->pairs.data(), b->pairs.size() * sizeof(PairRec));
+  if (e == cudaSuccess) e = upload(b->stream, b->d_pp, pp.data(), pp.size() * sizeof(PrimPair));
+  if (e == cudaSuccess) e = upload(b->stream, b->d_boys, ctxs[0]->d_boys, n_boys * 8, cudaMemcpyDeviceToDevice);
+  if (e == cudaSuccess) e = upload(b->stream, b->d_sph, ctxs[0]->d_sph, kSphTableDoubles * 8, cudaMemcpyDeviceToDevice);
+  if (e == cudaSuccess) e = upload(b->stream, b->d_offsets, offs.data(), offs.size() * 8);
+  if (e == cudaSuccess) e = upload(b->stream, b->d_dims, dims.data(), dims.size() * 4);
+  if (e == cudaSuccess) e = upload(b->stream, b->d_wmap_i, ints.data(), ints.size() * 4);
+  if (e == cudaSuccess && !cs.empty()) e = upload(b->stream, b->d_wmap_c, cs.data(), cs.size() * 8);
+  if (e == cudaSuccess && npair) e = upload(b->stream, b->d_row_bra, b->row_bra.data(), npair * 4);
+  if (e == cudaSuccess && npair) e = upload(b->stream, b->d_ks_i, ki.data(), npair * sizeof(int4));
+  if (e == cudaSuccess && npair) e = upload(b->stream, b->d_ks_q, kq.data(), npair * 8);
+  if (e == cudaSuccess && npair) e = upload(b->stream, b->d_ks_pp, kp.data(), 11 * npair * 8);
+  if (e == cudaSuccess) e = upload(b->stream, b->d_fine, ctxs[0]->d_fine, n_fine * 8, cudaMemcpyDeviceToDevice);
+  if (e == cudaSuccess) e = upload(b->stream, b->d_bsh, bsh.data(), bsh.size() * 4);
+  if (e == cudaSuccess) e = upload(b->stream, b->d_bmol, bmol.data(), bmol.size() * 4);
+  if (e == cudaSuccess) e = upload(b->stream, b->d_bpref, bpref.data(), bpref.size() * 8);
   for (int k = 0; k < dgf_batch::kBatchStreams; ++k) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->aux[k], cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join[k], cudaEventDisableTiming);
@@ -448,7 +448,7 @@ static int batch_plan(dgf_batch *b, double thrs) {
       cudaGetLastError();
       BFAIL(DGF_ERR_NOMEM, "device allocation of the batch plan failed");
     }
-    if (cudaMemcpy(b->d_row_tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess)
+    if (upload(b->stream, b->d_row_tasks, tasks.data(), tasks.size() * sizeof(int4)) != cudaSuccess)
       BFAIL(DGF_ERR_CUDA, "upload of the batch plan failed");
   }
   if (cudaMalloc(&b->d_qoff, std::max<size_t>(qoff.size(), 1) * 8) != cudaSuccess ||
@@ -456,8 +456,8 @@ static int batch_plan(dgf_batch *b, double thrs) {
     cudaGetLastError();
     BFAIL(DGF_ERR_NOMEM, "device allocation of the batch plan failed");
   }
-  if (cudaMemcpy(b->d_qoff, qoff.data(), qoff.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
-      (kbase.size() && cudaMemcpy(b->d_kbase, kbase.data(), kbase.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess))
+  if (upload(b->stream, b->d_qoff, qoff.data(), qoff.size() * 8) != cudaSuccess ||
+      (kbase.size() && upload(b->stream, b->d_kbase, kbase.data(), kbase.size() * 4) != cudaSuccess))
     BFAIL(DGF_ERR_CUDA, "upload of the batch plan failed");
   b->plan.swap(plan);
   b->plan_thrs = thrs;

@@ -232,6 +232,18 @@ inline dgf::WorkMaps ctx_maps(const dgf_ctx *c) {
   return m;
 }
 
+// A copy to the device on one of the library's streams, and a wait for it.
+// cudaMemcpy may return with the data still on its way (staged from pageable
+// memory, or device to device), and only the legacy stream and those that wait
+// for it run after it: the library's streams are non-blocking, and so may the
+// caller's be.  (Waiting for the legacy stream would do, but takes 0.5 ms in a
+// process with some thousand streams.)
+inline cudaError_t upload(cudaStream_t st, void *dst, const void *src, size_t bytes,
+                          cudaMemcpyKind kind = cudaMemcpyHostToDevice) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 struct DeviceGuard {
   int prev = -1;
   explicit DeviceGuard(int dev) {

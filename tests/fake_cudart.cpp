@@ -11,6 +11,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <set>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -29,6 +30,17 @@ long g_fail_malloc = -1, g_fail_malloc_n = 0;  // the calls [first, first + n) f
 int g_fail_instantiate = 0;
 cudaStream_t g_capturing = nullptr;  // the captured origin stream
 bool g_user_capture = false;
+struct Copy {
+  const char *dst;
+  cudaStream_t st;
+};
+std::vector<Copy> g_pending;                               // copies to the device that may not have landed
+std::map<cudaEvent_t, cudaStream_t> g_recorded;            // where an event was recorded last
+std::map<cudaStream_t, std::set<cudaStream_t>> g_waits;    // stream -> those whose work it waited for
+struct Range {
+  const char *begin, *end;
+};
+std::vector<Range> g_busy;  // what launches that may still run read
 cudaError_t g_last = cudaSuccess;
 // A captured launch of a quartet kernel, checked and counted at each replay.
 struct Launch {
@@ -56,6 +68,11 @@ bool live(const void *p, size_t n) {
   return (const char *)p + n <= it->first + it->second;
 }
 
+const char *block(const void *p) {  // the allocation p lies in
+  auto it = g_alloc.upper_bound((const char *)p);
+  return it == g_alloc.begin() ? nullptr : std::prev(it)->first;
+}
+
 void bad(const std::string &name, const char *what) { g_bad.push_back(name + ": " + what); }
 
 // Quartets of a launch of one of the Fock kernels.
@@ -75,6 +92,7 @@ void jk_launch(const std::string &name, const dgf::JKArgs &a, int nchunk) {
       break;
     }
   if (!live(a.bra, a.nbra * sizeof(PairRec))) return bad(name, "bra pairs");
+  auto reads = [](const void *q, size_t n) { g_busy.push_back({(const char *)q, (const char *)q + n}); };
   const bool same = a.same_class;
   const unsigned long long cls = ((l[0] * 4 + l[1]) * 4 + l[2]) * 4 + l[3];
   auto cover = [&](int ib, int ic) {
@@ -85,6 +103,7 @@ void jk_launch(const std::string &name, const dgf::JKArgs &a, int nchunk) {
   if (name.find("jk_row") != std::string::npos || name.find("jk_pack") != std::string::npos) {
     if (!live(a.row_tasks + a.row_task0, (a.row_task1 - a.row_task0) * sizeof(int4))) return bad(name, "row tasks");
     if (!live(a.row_work, nchunk * sizeof(unsigned))) return bad(name, "task counters");
+    reads(a.row_tasks + a.row_task0, (a.row_task1 - a.row_task0) * sizeof(int4));
     for (int t = a.row_task0; t < a.row_task1; ++t) {
       const int4 tk = a.row_tasks[t];
       const int nb = tk.y & 0xffff, kend = std::min(tk.w, tk.z + 32 * (tk.y >> 16));
@@ -98,6 +117,7 @@ void jk_launch(const std::string &name, const dgf::JKArgs &a, int nchunk) {
   }
   if (!live(a.qoff, (a.nbra + 1) * sizeof(int64_t))) return bad(name, "prefix sums");
   if (a.qoff[a.nbra] < a.nquartet) return bad(name, "prefix sums of another plan");
+  reads(a.qoff, (a.nbra + 1) * sizeof(int64_t));
   for (int ib = 0; ib < a.nbra; ++ib)
     for (int64_t q = std::max(a.qoff[ib], a.q_begin); q < std::min(a.qoff[ib + 1], a.nquartet); ++q) {
       const int ic = (int)(q - a.qoff[ib]);
@@ -171,16 +191,36 @@ cudaError_t cudaFree(void *p) {
     g_bad.push_back("cudaFree of a pointer that is not live");
     return ret(cudaErrorInvalidValue);
   }
+  g_busy.clear();  // waits for the device
   free(p);
   return cudaSuccess;
 }
-cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
+// From pageable memory cudaMemcpy returns once the data is staged, and between
+// device buffers at once: kernels on streams that do not wait for the legacy
+// stream may find the old contents.
+static void copied(void *d, size_t n, cudaMemcpyKind kind, cudaStream_t st) {
+  if (kind == cudaMemcpyDeviceToHost || !n) return;
+  for (const Range &r : g_busy)
+    if ((const char *)d < r.end && (const char *)d + n > r.begin) {
+      g_bad.push_back("a copy over what a running build reads");
+      break;
+    }
+  g_pending.push_back({(const char *)d, st});
+}
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind kind) {
   if (g_user_capture) return ret(cudaErrorStreamCaptureUnsupported);
   if (n) memcpy(d, s, n);
+  copied(d, n, kind, nullptr);
   return cudaSuccess;
 }
-cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) {
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind kind, cudaStream_t st) {
   if (n) memcpy(d, s, n);
+  copied(d, n, kind, st);
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceSynchronize() {
+  g_busy.clear();
+  g_pending.clear();
   return cudaSuccess;
 }
 cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t) {
@@ -199,12 +239,19 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) {
   free(s);
   return cudaSuccess;
 }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+  g_pending.erase(std::remove_if(g_pending.begin(), g_pending.end(), [s](const Copy &c) { return c.st == s; }),
+                  g_pending.end());
+  return cudaSuccess;
+}
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
+  g_waits[s].insert(g_recorded[e]);
+  return cudaSuccess;
+}
 cudaError_t cudaEventCreate(cudaEvent_t *e) { return *e = (cudaEvent_t)malloc(8), cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return *e = (cudaEvent_t)malloc(8), cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { return free(e), cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { return g_recorded[e] = s, cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { return *ms = 1.f, cudaSuccess; }
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus *c) {
@@ -237,12 +284,18 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t x) { return delete (Graph *)x, 
 cudaError_t cudaGetSymbolAddress(void **p, const void *s) { return *p = (void *)s, cudaSuccess; }
 cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }
 
-cudaError_t cudaLaunchKernel(const void *f, dim3 grid, dim3, void **args, size_t, cudaStream_t) {
+cudaError_t cudaLaunchKernel(const void *f, dim3 grid, dim3, void **args, size_t, cudaStream_t st) {
   ++g_launches;
   const auto it = g_kernel.find(f);
   if (it == g_kernel.end()) return ret(cudaErrorInvalidDeviceFunction);
   if (it->second.find("jk_") != std::string::npos && it->second.find("JKArgs") != std::string::npos) {
     const dgf::JKArgs &a = *(const dgf::JKArgs *)args[0];
+    const void *reads[] = {a.bra,  a.ket,  a.pp,   a.boys,  a.sph,       a.qoff,    a.blk_gab,
+                           a.ks_i, a.ks_q, a.ks_pp, a.row_bra, a.row_tasks, a.boys_fine};
+    for (const Copy &c : g_pending)
+      for (const void *r : reads)
+        if (c.st != st && !g_waits[st].count(c.st) && r && block(r) == block(c.dst))
+          g_bad.push_back(it->second + ": on a stream that does not wait for an upload");
     if (g_capturing)
       g_recording.push_back(Launch{it->second, a, (int)grid.y});
     else

@@ -268,3 +268,42 @@ def test_build_without_a_graph(host):
     for x in r["res"]:
         assert x[:4] == [0, r["res"][0][1], 0, ""] and x[5] == r["res"][0][5], r["res"]
     assert [x[4] for x in r["res"]] == [0, 0, 0, 0, 0, 1, 1, 1]
+
+
+@pytest.mark.parametrize("basis", ["cc-pVDZ", "6-31G*", "cc-pVTZ"])
+def test_launches_wait_for_uploads(host, basis):
+    """No kernel runs on one of the library's own streams, which do not wait
+    for the legacy stream, while a cudaMemcpy may still be on its way to the
+    device; and no plan is replaced while a build on another stream may still
+    read it."""
+    r = host(f"""
+    from dalton_b200.batch import BatchBuilder
+    F.fake_reset()
+    fb = builder({basis!r})
+    res = dict(create=F.fake_bad().decode())
+    for name, call in dict(
+            count=lambda: fb.ao_quartets(1e-6), fock=lambda: fb.herfck(eye(fb), thrs=1e-6),
+            screened=lambda: fb.herfck(eye(fb), thrs=1e-6, ifthrs=10), one=lambda: fb.oneint(),
+            grad=lambda: fb.grad2e(eye(fb)) if {basis!r} != "cc-pVTZ" else None).items():
+        F.fake_reset()
+        call()
+        res[name] = F.fake_bad().decode()
+    lib, ift, stream = _lib.load(), (_lib.dgf_int * 1)(13), np.zeros(1)
+    buf = np.zeros((2, fb.nbf, fb.nbf))
+    F.fake_reset()
+    for t in (1e-6, 1e-2, 1e-6, 1e-4):  # asynchronous builds on the caller's stream, one plan after the other
+        opt = _lib.default_options(thrs=t)
+        assert lib.dgf_fock_device(fb._h, 1, ift, buf[0].ctypes.data, buf[1].ctypes.data, ctypes.byref(opt),
+                                   stream.ctypes.data, None) == 0
+    res["plans"] = F.fake_bad().decode()
+    F.fake_reset()
+    bb = BatchBuilder([fb, builder({basis!r}, 2)])
+    p = np.zeros(2 * bb.total)
+    for t in (1e-4, 1e-2, 1e-4):
+        opt = _lib.default_options(thrs=t)
+        assert lib.dgf_fock_batch(bb._h, p.ctypes.data, p.ctypes.data + 8 * bb.total, ctypes.byref(opt), 0,
+                                  stream.ctypes.data, None) == 0
+    res["batch"] = F.fake_bad().decode()
+    out(**res)
+    """)
+    assert r == {k: "" for k in r}
