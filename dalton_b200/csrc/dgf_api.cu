@@ -153,6 +153,11 @@ void boys_fine_host(std::vector<double> &out) {
   }
 }
 
+const std::vector<double> &boys_fine_table() {
+  static const std::vector<double> t = [] { std::vector<double> v; boys_fine_host(v); return v; }();
+  return t;
+}
+
 // Cartesian -> real spherical coefficients with Dalton's conventions (SPHCO1,
 // DALTON/abacus/her1pro.F:4697-4770, MORDER=1 so m = -l..l, MINTEG=2 so the
 // functions are normalised given Cartesians carrying the x^l norm), from the
@@ -895,28 +900,20 @@ static int create_ctx(const dgf_basis *b, int device, bool resolve_all, dgf_ctx 
   DGF_CUDA_CHECK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   DGF_CUDA_CHECK(cudaEventCreate(&c->ev0));
   DGF_CUDA_CHECK(cudaEventCreate(&c->ev1));
-  DGF_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
-  for (int k = 1; k < kForkStreams; ++k) {
-    DGF_CUDA_CHECK(cudaStreamCreateWithFlags(&c->fork[k], cudaStreamNonBlocking));
-    DGF_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_join[k], cudaEventDisableTiming));
-  }
   DGF_CUDA_CHECK(jk_prepare_all());
   // the Boys tables hold constants only: made once per process
   static const std::vector<double> boys = [] { std::vector<double> v; boys_table_host(v); return v; }();
-  static const std::vector<double> fine = [] { std::vector<double> v; boys_fine_host(v); return v; }();
   std::vector<double> sph;
   sph_table_host(sph);
   if (dev_alloc(&c->d_boys, boys.size()) != cudaSuccess || dev_alloc(&c->d_sph, sph.size()) != cudaSuccess ||
       dev_alloc(&c->d_pp, c->pp.size()) != cudaSuccess || dev_alloc(&c->d_pairs, c->pairs.size()) != cudaSuccess ||
-      dev_alloc(&c->d_cnt, 4 * kCounterSlots) != cudaSuccess || dev_alloc(&c->d_fine, fine.size()) != cudaSuccess ||
-      dev_alloc(&c->d_row_bra, c->pairs.size()) != cudaSuccess ||
-      dev_alloc(&c->d_row_work, (size_t)kRowSlots * kRowChunksMax) != cudaSuccess) {
+      dev_alloc(&c->d_cnt, 4 * kCounterSlots) != cudaSuccess ||
+      dev_alloc(&c->d_row_bra, c->pairs.size()) != cudaSuccess) {
     cudaGetLastError();
     DGF_FAIL(DGF_ERR_NOMEM, "device allocation failed while creating the context");
   }
   DGF_CUDA_CHECK(upload(c->stream, c->d_boys, boys.data(), boys.size() * 8));
   DGF_CUDA_CHECK(upload(c->stream, c->d_sph, sph.data(), sph.size() * 8));
-  DGF_CUDA_CHECK(upload(c->stream, c->d_fine, fine.data(), fine.size() * 8));
   DGF_CUDA_CHECK(upload(c->stream, c->d_pp, c->pp.data(), c->pp.size() * sizeof(PrimPair)));
   DGF_CUDA_CHECK(
       upload(c->stream, c->d_pairs, c->pairs.data(), c->pairs.size() * sizeof(PairRec)));
@@ -1198,8 +1195,35 @@ static int ensure_frags(dgf_ctx *c, const std::vector<ClassPlan> &plan) {
   return DGF_OK;
 }
 
+// What a context's own launches need besides its pairs: the forked streams and
+// their events, the row kernels' Boys table and task counters.  Made with the
+// first plan: a context that only takes part in batches never has them (a
+// stream holds over half a megabyte of device memory).
+static int ensure_launch_state(dgf_ctx *c) {
+  if (!c->ev_fork) DGF_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+  for (int k = 1; k < kForkStreams; ++k) {
+    if (!c->fork[k]) DGF_CUDA_CHECK(cudaStreamCreateWithFlags(&c->fork[k], cudaStreamNonBlocking));
+    if (!c->ev_join[k]) DGF_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_join[k], cudaEventDisableTiming));
+  }
+  if (c->d_fine) return DGF_OK;
+  const std::vector<double> &fine = boys_fine_table();
+  double *p = nullptr;
+  if (!c->d_row_work && dev_alloc(&c->d_row_work, (size_t)kRowSlots * kRowChunksMax) != cudaSuccess)
+    c->d_row_work = nullptr;
+  if (!c->d_row_work || dev_alloc(&p, fine.size()) != cudaSuccess) {
+    cudaGetLastError();
+    DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the row kernels' tables failed");
+  }
+  const cudaError_t e = upload(c->stream, p, fine.data(), fine.size() * 8);
+  if (e != cudaSuccess) cudaFree(p);
+  DGF_CUDA_CHECK(e);
+  c->d_fine = p;
+  return DGF_OK;
+}
+
 static int build_plan(dgf_ctx *c, double thrs) {
   if (c->plan_thrs == thrs && !c->plan.empty()) return DGF_OK;
+  if (const int r = ensure_launch_state(c)) return r;
   std::vector<int64_t> all;
   std::vector<ClassPlan> plan;
   std::vector<int4> tasks;

@@ -312,7 +312,7 @@ extern "C" int dgf_batch_create(dgf_ctx *const *caller_ctxs, dgf_int nmol, dgf_b
   if (e == cudaSuccess && npair) e = upload(b->stream, b->d_ks_i, ki.data(), npair * sizeof(int4));
   if (e == cudaSuccess && npair) e = upload(b->stream, b->d_ks_q, kq.data(), npair * 8);
   if (e == cudaSuccess && npair) e = upload(b->stream, b->d_ks_pp, kp.data(), 11 * npair * 8);
-  if (e == cudaSuccess) e = upload(b->stream, b->d_fine, ctxs[0]->d_fine, n_fine * 8, cudaMemcpyDeviceToDevice);
+  if (e == cudaSuccess) e = upload(b->stream, b->d_fine, boys_fine_table().data(), n_fine * 8);
   if (e == cudaSuccess) e = upload(b->stream, b->d_bsh, bsh.data(), bsh.size() * 4);
   if (e == cudaSuccess) e = upload(b->stream, b->d_bmol, bmol.data(), bmol.size() * 4);
   if (e == cudaSuccess) e = upload(b->stream, b->d_bpref, bpref.data(), bpref.size() * 8);

@@ -234,6 +234,7 @@ cudaError_t jk_prepare_all();
 
 void boys_table_host(std::vector<double> &out);       // [kBoysMaxM+1][kBoysTableDoubles]
 void boys_fine_host(std::vector<double> &out);        // [kFineMaxM+1][kFineDoubles]
+const std::vector<double> &boys_fine_table();         // the same, made once per process
 void sph_table_host(std::vector<double> &out);        // kSphTableDoubles
 double boys_reference(int m, double t);               // accurate host F_m(t)
 

@@ -307,3 +307,33 @@ def test_launches_wait_for_uploads(host, basis):
     out(**res)
     """)
     assert r == {k: "" for k in r}
+
+
+@pytest.mark.parametrize("basis", ["cc-pVDZ", "6-31G*"])
+def test_contexts_of_a_batch_stay_small(host, basis):
+    """A context makes its launch streams and tables with its first plan: one
+    that only takes part in batches holds its own stream and no more, nor does
+    its resolved form."""
+    r = host(f"""
+    from dalton_b200.batch import BatchBuilder
+    fbs = [builder({basis!r}, n) for n in (1, 2, 1)]
+    made = F.fake_streams()
+    bb = BatchBuilder(fbs)
+    batch = F.fake_streams() - made
+    live = F.fake_live()
+    F.fake_reset()
+    fbs[0].herfck(eye(fbs[0]), thrs=1e-6)
+    first = F.fake_streams() - made - batch
+    fbs[0].herfck(eye(fbs[0]), thrs=1e-4)
+    fbs[0].grad2e(eye(fbs[0]))
+    later = F.fake_streams() - made - batch - first
+    bb.close()
+    for fb in fbs:
+        fb.close()
+    out(made=made, batch=batch, first=first, later=later, left=[F.fake_streams(), F.fake_live()], bad=F.fake_bad().decode())
+    """)
+    forms = 2 if basis == "6-31G*" else 1
+    assert r["made"] == 3
+    assert r["batch"] == 5 + 3 * (forms - 1)  # its own five, and one of each resolved form
+    assert (r["first"], r["later"]) == (7, 0)
+    assert r["left"] == [0, 0] and r["bad"] == ""
