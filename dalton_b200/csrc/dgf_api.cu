@@ -184,7 +184,7 @@ static void free_ctx(dgf_ctx *c) {
                   c->d_dmax,  c->d_cnt,    c->d_qoff,   c->d_wmap_i, c->d_wmap_c, c->d_wmeta, c->d_wdims, c->d_gw,
                   c->d_shinfo, c->d_blk_gab, c->d_blk_info, c->d_blk_dmax, c->d_ks_i, c->d_ks_q, c->d_ks_pp,
                   c->d_store, c->d_fine,   c->d_row_bra, c->d_row_tasks, c->d_row_work,
-                  c->d_one,   c->d_pg,    c->d_one_pairs, c->d_one_pp};
+                  c->d_one,   c->d_pg,    c->d_far,   c->d_far_pp};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (double *p : c->d_frag)
@@ -489,10 +489,11 @@ struct ShellList {
 };
 
 // Shell pairs A >= B (the higher l first) with their primitive pairs, class
-// by class; primitive pairs with mu |AB|^2 > reach are dropped.  The
+// by class, of the primitive pairs with near < mu |AB|^2 <= far.  The
 // two-electron lists stop at 40 (e^-40 ~ 4e-18).
+constexpr double kPairReach = 40.0;
 static void build_pairs(const dgf_ctx *c, const ShellList &sh, int nbfm, std::vector<PairRec> &pairs,
-                        int *cls_off, std::vector<PrimPair> &pp, double reach = 40.0) {
+                        int *cls_off, std::vector<PrimPair> &pp, double near = -1.0, double far = kPairReach) {
   const double r2pi52 = std::sqrt(2.0 * std::pow(3.14159265358979323846, 2.5));
   std::vector<std::vector<PairRec>> bycls(kNumPairClass);
   pp.clear();
@@ -524,7 +525,7 @@ static void build_pairs(const dgf_ctx *c, const ShellList &sh, int nbfm, std::ve
         for (int j = 0; j < sh.nprim[sb]; ++j) {
           const double ea = sh.a[sh.p0[sa] + i], eb = sh.a[sh.p0[sb] + j];
           const double p = ea + eb, mu = ea * eb / p;
-          if (mu * ab2 > reach) continue;
+          if (mu * ab2 > far || !(mu * ab2 > near)) continue;
           PrimPair q;
           q.p = p;
           q.Px = (ea * xa[0] + eb * xb[0]) / p;
@@ -551,32 +552,28 @@ static void build_pairs(const dgf_ctx *c, const ShellList &sh, int nbfm, std::ve
   }
 }
 
-// The pair list of the one-electron calls: all primitive pairs up to
-// x = mu |AB|^2 = 80, where the two-electron lists stop at 40.  A pair of
-// normalised primitives has |S| <= (4 x)^{(la + lb)/2} e^-x, T and the
-// derivatives further powers of x: above 1e-12 with f shells at x = 40 (two
-// carbon atoms in cc-pVTZ, Cartesian: S 2e-12, T 4e-11, gradient 5e-12),
-// below 1e-22 at x = 80.  Pairs with most primitives first, so that a warp's
-// lanes have about as many each.
-constexpr double kOneReach = 80.0;
-int one_pairs(dgf_ctx *c) {
-  if (c->one_made) return DGF_OK;
+// The primitive pairs of the one-electron calls beyond the two-electron lists:
+// x = mu |AB|^2 from 40 to 80.  A pair of normalised primitives has
+// |S| <= (4 x)^{(la + lb)/2} e^-x, T and the derivatives further powers of x:
+// above 1e-12 with f shells at x = 40 (two carbon atoms in cc-pVTZ, Cartesian:
+// S 2e-12, T 4e-11, gradient 5e-12), below 1e-22 at x = 80.
+constexpr double kFarReach = 80.0;
+int far_pairs(dgf_ctx *c) {
+  if (c->far_made) return DGF_OK;
   std::vector<PairRec> pairs;
   std::vector<PrimPair> pp;
   build_pairs(c, ShellList{c->ws_l, c->ws_atom, c->ws_ao, c->ws_nprim, c->ws_p0, c->ws_a, c->ws_c, &c->ws_blk_flag},
-              c->nwf, pairs, c->one_off, pp, kOneReach);
-  for (int X = 0; X < kNumPairClass; ++X)
-    std::stable_sort(pairs.begin() + c->one_off[X], pairs.begin() + c->one_off[X + 1],
-                     [](const PairRec &u, const PairRec &v) { return u.npp > v.npp; });
-  if (!c->d_one_pairs && dev_alloc(&c->d_one_pairs, pairs.size()) != cudaSuccess) c->d_one_pairs = nullptr;
-  if (!c->d_one_pp && dev_alloc(&c->d_one_pp, pp.size()) != cudaSuccess) c->d_one_pp = nullptr;
-  if (!c->d_one_pairs || !c->d_one_pp) {
+              c->nwf, pairs, c->far_off, pp, kPairReach, kFarReach);
+  if (!c->d_far && dev_alloc(&c->d_far, pairs.size()) != cudaSuccess) c->d_far = nullptr;
+  if (!c->d_far_pp && dev_alloc(&c->d_far_pp, pp.size()) != cudaSuccess) c->d_far_pp = nullptr;
+  if (!c->d_far || !c->d_far_pp) {
     cudaGetLastError();
     DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the one-electron pairs failed");
   }
-  DGF_CUDA_CHECK(upload(c->stream, c->d_one_pairs, pairs.data(), pairs.size() * sizeof(PairRec)));
-  DGF_CUDA_CHECK(upload(c->stream, c->d_one_pp, pp.data(), pp.size() * sizeof(PrimPair)));
-  c->one_made = true;
+  DGF_CUDA_CHECK(upload(c->stream, c->d_far, pairs.data(), pairs.size() * sizeof(PairRec)));
+  DGF_CUDA_CHECK(upload(c->stream, c->d_far_pp, pp.data(), pp.size() * sizeof(PrimPair)));
+  DGF_CUDA_CHECK(cudaStreamSynchronize(c->stream));
+  c->far_made = true;
   return DGF_OK;
 }
 
@@ -735,8 +732,11 @@ extern "C" void dgf_default_options(dgf_options *opt) {
   opt->hfxatt = 0.0;
 }
 
-// Working functions a resolved context may have: the largest size every entry
-// point takes (dgf_fock_device_noalloc's fixed scratch).
+// Working functions a resolved context may have: the limit of
+// dgf_fock_device_noalloc's fixed scratch, so that it can run on the plan that
+// a context's other builds made.  The builds themselves would gain beyond it:
+// 43 waters in 6-31G* (1505 functions) take 93 ms resolved and 147 ms
+// contracted, 44 waters 156 ms contracted.
 constexpr int kPrimMaxW = 1536;
 
 // Keeps a copy of the basis where contracted shells could be resolved.
@@ -998,6 +998,7 @@ static int create_ctx(const dgf_basis *b, int device, bool resolve_all, dgf_ctx 
     DGF_CUDA_CHECK(upload(c->stream, c->d_ks_q, kq.data(), np * 8));
     DGF_CUDA_CHECK(upload(c->stream, c->d_ks_pp, kp.data(), 11 * np * 8));
   }
+  DGF_CUDA_CHECK(cudaStreamSynchronize(c->stream));
   *out = c.release();
   return DGF_OK;
 }
@@ -1214,7 +1215,7 @@ static int ensure_launch_state(dgf_ctx *c) {
     cudaGetLastError();
     DGF_FAIL(DGF_ERR_NOMEM, "device allocation of the row kernels' tables failed");
   }
-  const cudaError_t e = upload(c->stream, p, fine.data(), fine.size() * 8);
+  const cudaError_t e = upload(c->stream, p, fine.data(), fine.size() * 8);  // waited for with the plan
   if (e != cudaSuccess) cudaFree(p);
   DGF_CUDA_CHECK(e);
   c->d_fine = p;
@@ -1303,6 +1304,7 @@ static int build_plan(dgf_ctx *c, double thrs) {
   }
   DGF_CUDA_CHECK(upload(c->stream, c->d_qoff, all.data(), all.size() * 8));
   if (const int r = ensure_frags(c, plan)) return r;
+  DGF_CUDA_CHECK(cudaStreamSynchronize(c->stream));
   c->plan.swap(plan);
   c->plan_thrs = thrs;
   ++c->gen;
@@ -1433,6 +1435,7 @@ static int ensure_block_screen(dgf_ctx *c, int nslot) {
     }
     DGF_CUDA_CHECK(upload(c->stream, c->d_blk_gab, gab.data(), nb2 * 8));
     DGF_CUDA_CHECK(upload(c->stream, c->d_blk_info, info.data(), info.size() * sizeof(int)));
+    DGF_CUDA_CHECK(cudaStreamSynchronize(c->stream));
   }
   if (nslot > c->cap_blk_slots) {
     ++c->gen;

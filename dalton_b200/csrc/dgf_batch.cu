@@ -316,6 +316,7 @@ extern "C" int dgf_batch_create(dgf_ctx *const *caller_ctxs, dgf_int nmol, dgf_b
   if (e == cudaSuccess) e = upload(b->stream, b->d_bsh, bsh.data(), bsh.size() * 4);
   if (e == cudaSuccess) e = upload(b->stream, b->d_bmol, bmol.data(), bmol.size() * 4);
   if (e == cudaSuccess) e = upload(b->stream, b->d_bpref, bpref.data(), bpref.size() * 8);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
   for (int k = 0; k < dgf_batch::kBatchStreams; ++k) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->aux[k], cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join[k], cudaEventDisableTiming);
@@ -457,7 +458,8 @@ static int batch_plan(dgf_batch *b, double thrs) {
     BFAIL(DGF_ERR_NOMEM, "device allocation of the batch plan failed");
   }
   if (upload(b->stream, b->d_qoff, qoff.data(), qoff.size() * 8) != cudaSuccess ||
-      (kbase.size() && upload(b->stream, b->d_kbase, kbase.data(), kbase.size() * 4) != cudaSuccess))
+      (kbase.size() && upload(b->stream, b->d_kbase, kbase.data(), kbase.size() * 4) != cudaSuccess) ||
+      cudaStreamSynchronize(b->stream) != cudaSuccess)
     BFAIL(DGF_ERR_CUDA, "upload of the batch plan failed");
   b->plan.swap(plan);
   b->plan_thrs = thrs;

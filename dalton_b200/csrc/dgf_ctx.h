@@ -99,11 +99,11 @@ struct dgf_ctx {
   int64_t *d_wmeta = nullptr;   // {0, nwf^2} {0, nbf^2} element offsets of the single-molecule form
   int *d_wdims = nullptr;       // {nwf, nbf, 0, 0}
   double *d_one = nullptr;      // scratch of the one-electron calls (dgf_grad.cu), made by the first of them
-  // their pairs, by class (one_pairs)
-  bool one_made = false;
-  int one_off[dgf::kNumPairClass + 1] = {0};
-  dgf::PairRec *d_one_pairs = nullptr;
-  dgf::PrimPair *d_one_pp = nullptr;
+  // their primitive pairs beyond the two-electron lists, by class (far_pairs)
+  bool far_made = false;
+  int far_off[dgf::kNumPairClass + 1] = {0};
+  dgf::PairRec *d_far = nullptr;
+  dgf::PrimPair *d_far_pp = nullptr;
   double *d_pg = nullptr;       // two-electron gradient: derivatives per pair (6 each), then task counters
   double *d_gw = nullptr;       // working-basis densities of the two-electron gradient (2 nwf^2)
   int *d_shinfo = nullptr;      // per working shell: first function | function count (density bounds)
@@ -168,8 +168,9 @@ struct dgf_ctx {
   cudaEvent_t ev_fork = nullptr, ev_join[kForkStreams] = {};
   std::vector<dgf_graph> graphs;
   int64_t gen = 0, graph_gen = 0;  // counts changes of plan, buffers and kernel choices; of the kept graphs
-  // kernel choice per class pair and precision (-5 = row kernel, -1 = team
-  // kernel, >= 0 = thread-kernel variant), set by the autotuner;
+  // kernel choice per class pair and precision (-6 = pack kernel, -5 = row
+  // kernel, -4 and -3 = warp kernels, -2 and -1 = team kernels, >= 0 =
+  // thread-kernel variant), set by the autotuner;
   // kDefaultVariant by default
   int choice[dgf::kNumPairClass][dgf::kNumPairClass][2] = {};
   // mixed form: whether a class pair is split into FP64 and FP32 launches
@@ -193,8 +194,8 @@ struct RowSource {
   const int64_t *qoff;
   int bra0, ket0, ket_end;
 };
-// Makes the pair list of a context's one-electron calls (dgf_api.cu).
-int one_pairs(dgf_ctx *c);
+// Makes the far pairs of a context's one-electron calls (dgf_api.cu).
+int far_pairs(dgf_ctx *c);
 
 // Appends the row tasks of a launch (dgf_api.cu).
 void row_tasks(const std::vector<RowSource> &src, int max_bras, int min_width, std::vector<int4> &tasks);
@@ -232,16 +233,16 @@ inline dgf::WorkMaps ctx_maps(const dgf_ctx *c) {
   return m;
 }
 
-// A copy to the device on one of the library's streams, and a wait for it.
-// cudaMemcpy may return with the data still on its way (staged from pageable
-// memory, or device to device), and only the legacy stream and those that wait
-// for it run after it: the library's streams are non-blocking, and so may the
-// caller's be.  (Waiting for the legacy stream would do, but takes 0.5 ms in a
-// process with some thousand streams.)
+// A copy to the device on one of the library's streams.  Work on other streams
+// may use it once that stream has been waited for: every function that uploads
+// ends with that wait, except for what only the same stream reads before.
+// cudaMemcpy does not do: it may return with the data still on its way (staged
+// from pageable memory, or device to device), and only the legacy stream and
+// those that wait for it run after it, while the library's streams are
+// non-blocking, and so may the caller's be.
 inline cudaError_t upload(cudaStream_t st, void *dst, const void *src, size_t bytes,
                           cudaMemcpyKind kind = cudaMemcpyHostToDevice) {
-  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, st);
-  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+  return cudaMemcpyAsync(dst, src, bytes, kind, st);
 }
 
 struct DeviceGuard {

@@ -3,9 +3,9 @@
 // (HER1INT, DALTON/abacus/her1drv.F; the operators' derivative integrals,
 // DALTON/abacus/aba1mat.F).
 //
-// Both work on the shell pairs of the two-electron working basis, in a list of
-// their own that reaches further (one_pairs), class by class with compile-time
-// angular momenta: one thread per pair, everything in registers for s, p and d
+// Both work on the shell pairs of the two-electron working basis and on the
+// primitive pairs that its lists leave out (far_pairs), class by class with
+// compile-time angular momenta: one thread per pair, everything in registers for s, p and d
 // shells, so that no index arithmetic or local memory stands between the Boys
 // functions.  A general contraction's primitives are evaluated once and mapped
 // to the AO basis afterwards (S = C^T S_w C; D_w = C D C^T).  The nuclear
@@ -35,9 +35,11 @@ constexpr double kInvR2Pi52 = 0.16906264579104438;  // 1 / sqrt(2 pi^(5/2))
 constexpr int kOneBlock = 128;
 
 struct OneArgs {
-  const PairRec *pairs;  // one class
-  const PrimPair *pp;
-  int npair;
+  // one class: its two-electron list, then its far pairs (far_pairs); a
+  // contracted pair may be in both
+  const PairRec *pairs, *far;
+  const PrimPair *pp, *far_pp;
+  int nnear, npair;
   const double *xyz, *charge;  // nuclei
   int natom, nwf;
   const double *boys;    // table of the order this launch needs
@@ -102,12 +104,14 @@ __global__ void __launch_bounds__(kOneBlock) oneint_kernel(const OneArgs a) {
   for (int i = threadIdx.x; i < kBoysTableDoubles; i += blockDim.x) tab[i] = a.boys[i];
   __syncthreads();
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < a.npair; e += gridDim.x * blockDim.x) {
-    const PairRec pr = load_pair(a.pairs + e);
+    const bool far = e >= a.nnear;
+    const PairRec pr = load_pair(far ? a.far + (e - a.nnear) : a.pairs + e);
+    const PrimPair *pp = (far ? a.far_pp : a.pp) + pr.pp0;
     double S[NA * NB], T[NA * NB], V[NA * NB];
 #pragma unroll
     for (int k = 0; k < NA * NB; ++k) S[k] = T[k] = V[k] = 0.0;
     for (int m = 0; m < pr.npp; ++m) {
-      const PrimPair P = load_prim<true>(a.pp + pr.pp0 + m);
+      const PrimPair P = load_prim<true>(pp + m);
       const double eb = P.p - P.ea, h = 0.5 / P.p, kab = P.K * P.p * kInvR2Pi52;
       {
         double sx[(LA + 1) * (LB + 3)], sy[(LA + 1) * (LB + 3)], sz[(LA + 1) * (LB + 3)];
@@ -179,7 +183,7 @@ __global__ void __launch_bounds__(kOneBlock) oneint_kernel(const OneArgs a) {
         for (int k = 0; k < FA * FB; ++k) f[k] = c[k];
       }
 #pragma unroll
-      for (int k = 0; k < FA * FB; ++k) M[(size_t)(pr.aoA + k / FB) * a.nwf + pr.aoB + k % FB] = w * f[k];
+      for (int k = 0; k < FA * FB; ++k) atomicAdd(M + (size_t)(pr.aoA + k / FB) * a.nwf + pr.aoB + k % FB, w * f[k]);
     };
     put(a.S, S);
     put(a.T, T);
@@ -208,7 +212,10 @@ __global__ void __launch_bounds__(kOneBlock) grad1e_kernel(const OneArgs a) {
   const int stride = gridDim.x * blockDim.x;
   for (int e0 = blockIdx.x * blockDim.x + warp * 32; e0 < a.npair; e0 += stride) {
     const bool in = e0 + lane < a.npair;
-    const PairRec pr = load_pair(a.pairs + (in ? e0 + lane : a.npair - 1));
+    const int e = in ? e0 + lane : a.npair - 1;
+    const bool far = e >= a.nnear;
+    const PairRec pr = load_pair(far ? a.far + (e - a.nnear) : a.pairs + e);
+    const PrimPair *pp = (far ? a.far_pp : a.pp) + pr.pp0;
     const bool work = in && !(SWAP && pr.same);
     double D[NI * NJ], W[NI * NJ];
     grad::cart_block<LI, LJ, SPH>(a.D, a.nwf, SWAP ? pr.aoB : pr.aoA, SWAP ? pr.aoA : pr.aoB, D);
@@ -217,7 +224,7 @@ __global__ void __launch_bounds__(kOneBlock) grad1e_kernel(const OneArgs a) {
     const int nmax = __reduce_max_sync(0xffffffffu, work ? pr.npp : 0);
     for (int m = 0; m < nmax; ++m) {
       const bool on = work && m < pr.npp;
-      const PrimPair P = load_prim<true>(a.pp + pr.pp0 + (on ? m : 0));
+      const PrimPair P = load_prim<true>(pp + (on ? m : 0));
       const double ea = SWAP ? P.p - P.ea : P.ea, eb = P.p - ea, h = 0.5 / P.p;
       const double kab = on ? 2.0 * P.K * P.p * kInvR2Pi52 : 0.0;
       const double PI[3] = {SWAP ? P.PBx : P.PAx, SWAP ? P.PBy : P.PAy, SWAP ? P.PBz : P.PAz};
@@ -428,12 +435,22 @@ struct OneScratch {
 OneArgs one_args(const dgf_ctx *c, const OneScratch &s) {
   OneArgs a;
   memset(&a, 0, sizeof(a));
-  a.pp = c->d_one_pp;
+  a.pp = c->d_pp;
+  a.far_pp = c->d_far_pp;
   a.xyz = s.xyz;
   a.charge = s.charge;
   a.natom = c->natom;
   a.nwf = c->nwf;
   return a;
+}
+
+// The pairs of class X; false: none.
+bool class_pairs(const dgf_ctx *c, int X, OneArgs &a) {
+  a.nnear = c->cls_off[X + 1] - c->cls_off[X];
+  a.npair = a.nnear + c->far_off[X + 1] - c->far_off[X];
+  a.pairs = c->d_pairs + c->cls_off[X];
+  a.far = c->d_far + c->far_off[X];
+  return a.npair > 0;
 }
 
 }  // namespace
@@ -446,7 +463,7 @@ extern "C" int dgf_oneint(dgf_ctx *c, double *S, double *T, double *V) {
   DeviceGuard g(c->device);
   OneScratch s(c);
   int r = s.open();
-  if (!r) r = one_pairs(c);
+  if (!r) r = far_pairs(c);
   if (r) return r;
   OneArgs a = one_args(c, s);
   a.S = S ? s.w : nullptr;
@@ -454,9 +471,7 @@ extern "C" int dgf_oneint(dgf_ctx *c, double *S, double *T, double *V) {
   a.V = V ? s.w + 2 * s.n2w : nullptr;
   cudaError_t e = cudaMemsetAsync(s.w, 0, 3 * s.n2w * 8);
   for (int X = 0; X < kNumPairClass && e == cudaSuccess; ++X) {
-    a.npair = c->one_off[X + 1] - c->one_off[X];
-    if (!a.npair) continue;
-    a.pairs = c->d_one_pairs + c->one_off[X];
+    if (!class_pairs(c, X, a)) continue;
     a.boys = c->d_boys + (size_t)kPairClassL[X] * kBoysTableDoubles;
     kOneint[X](a, c->spherical != 0, c->nsm);
     e = cudaGetLastError();
@@ -484,7 +499,7 @@ extern "C" int dgf_grad1e(dgf_ctx *c, const double *dmat, const double *wmat, do
   DeviceGuard g(c->device);
   OneScratch s(c);
   int r = s.open();
-  if (!r) r = one_pairs(c);
+  if (!r) r = far_pairs(c);
   if (r) return r;
   OneArgs a = one_args(c, s);
   cudaError_t e = cudaMemcpy(s.ao, dmat, s.n2 * 8, cudaMemcpyHostToDevice);
@@ -499,9 +514,7 @@ extern "C" int dgf_grad1e(dgf_ctx *c, const double *dmat, const double *wmat, do
   a.smem_acc = c->natom <= kOneSmemAtoms;
   if (e == cudaSuccess) e = cudaGetLastError();
   for (int X = 0; X < kNumPairClass && e == cudaSuccess; ++X) {
-    a.npair = c->one_off[X + 1] - c->one_off[X];
-    if (!a.npair) continue;
-    a.pairs = c->d_one_pairs + c->one_off[X];
+    if (!class_pairs(c, X, a)) continue;
     a.boys = c->d_boys + (size_t)(kPairClassL[X] + 1) * kBoysTableDoubles;
     kGrad1e[X](a, c->spherical != 0, c->nsm);
     e = cudaGetLastError();

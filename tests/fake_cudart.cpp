@@ -192,6 +192,7 @@ cudaError_t cudaFree(void *p) {
     return ret(cudaErrorInvalidValue);
   }
   g_busy.clear();  // waits for the device
+  g_pending.clear();
   free(p);
   return cudaSuccess;
 }
