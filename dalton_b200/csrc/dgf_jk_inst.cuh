@@ -1,11 +1,13 @@
 // The quartet-class kernel table of libdgfock and what its instantiation
-// units share.  The entry of class pair (X, Y) is filled by four generated
+// units share.  The entry of class pair (X, Y) is filled by five generated
 // translation units (parts) so that the heaviest classes compile in
 // parallel and a change to one kernel family rebuilds only its units:
 // part 0 the cooperative, warp-team and warp-per-quartet kernels
 // (dgf_jk_inst_team.cuh), parts 1 and 2 the FP64 and FP32 thread kernels
-// (dgf_jk_inst_thread.cuh), part 3 the row kernel (dgf_jk_inst_row.cuh).  Each part sets only its own fields of the
-// (zero-initialised) entry and its own prepare hook.
+// (dgf_jk_inst_thread.cuh), part 3 the row kernel (dgf_jk_inst_row.cuh), part
+// 4 the pack kernel (dgf_jk_inst_pack.cuh; its tables are in dgf_pack.h).  Each
+// part sets only its own fields of the (zero-initialised) entry and its own
+// prepare hook.
 #pragma once
 
 #include "dgf_internal.h"

@@ -12,11 +12,12 @@ namespace jkinst {
 constexpr bool pack_eligible(int LA, int LB, int LC, int LD) {
   return LA >= 2 && LA + LB + LC + LD >= 4 && (2 * LC + 1) * (2 * LD + 1) >= (LA == 3 ? 3 : 5);
 }
-// The default among them: f bras, where the row kernel has no form (L > 5).
-// On C5H12 / cc-pVTZ (ms per class): (fd|ps) 2.8 against 3.4 of the warp
-// kernel, (fp|ds) 1.7 / 2.8, (fd|dp) 1.4 / 3.3, (ff|fd) 1.6 / 3.0 (team),
-// (ff|ps) 0.55 / 1.9.  With d bras the warp kernel is faster ((dp|dp) of
-// (H2O)32 / cc-pVDZ 2.8 against 3.6) and has the FP32 half of the mixed form.
+// The default among them: L > 5, where the row kernel has no form.  Every such
+// class is faster than with the warp kernel (team kernel: *); ms per class on
+// C5H12 / cc-pVTZ: (fd|ps) 1.77 against 3.44, (dp|dp) 1.63 / 2.21, (fs|dp)
+// 1.46 / 1.80, (fp|ds) 1.39 / 2.77, (fd|dp) 1.00 / 3.32, (ff|ps) 0.35 / 1.85,
+// (ff|fd) 0.19 / 2.97*; on (H2O)32 / cc-pVDZ: (dd|pp) 2.01 / 2.09, (dp|dp)
+// 1.72 / 2.78, (dd|ds) 1.46 / 1.51, (dd|dp) 0.60 / 1.01, (dd|dd) 0.07 / 0.25.
 constexpr bool pack_preferred(int LA, int LB, int LC, int LD) { return LA + LB + LC + LD > 5; }
 
 template <int LA, int LB, int LC, int LD>

@@ -80,9 +80,10 @@ class FockBuilder:
 
     def set_class_kernel(self, cls, variant, precision=64):
         """Pin the kernel of quartet class ``cls`` = (la, lb, lc, ld): variant
-        -5 row kernel (FP64), -4 warp per quartet with FP64 tensor-core (DMMA) transforms, -3 warp
-        per quartet, -2 warp team, -1 cooperative team, 0.. thread chunk
-        variants."""
+        -6 pack kernel (FP64), -5 row kernel (FP64), -4 warp per quartet with
+        FP64 tensor-core (DMMA) transforms, -3 warp per quartet, -2 warp team,
+        -1 cooperative team, 0.. thread chunk variants.  A pinned context runs
+        its whole builds on its own pairs, also in a segmented basis."""
         la, lb, lc, ld = (int(x) for x in cls)
         _lib.check(self._lib.dgf_set_class_kernel(self._h, la, lb, lc, ld, int(precision), int(variant)),
                    "dgf_set_class_kernel")

@@ -74,9 +74,13 @@ typedef struct {
 /* Work counters of one call (HERFCK's DINTSKP/SCRSTA statistics,
  * her2drv.F:495-541, her2gab.F:1486, in this library's units: shell quartets
  * of the two-electron working basis, in which general contractions are
- * resolved into primitives; dgf_count_ao_quartets gives the AO-basis count). */
+ * resolved into primitives.  Direct builds, gradients and batches of a basis
+ * with segmented contractions resolve those too (up to 1536 primitive
+ * functions, until a kernel is pinned on the context): their counts are of
+ * primitive shell quartets with Q_AB*Q_CD >= 1e-3 thrs.
+ * dgf_count_ao_quartets gives the AO-basis count). */
 typedef struct {
-  int64_t quartets_total;    /* canonical shell quartets with Q_AB*Q_CD >= thrs */
+  int64_t quartets_total;    /* canonical shell quartets that pass the Schwarz screen */
   int64_t quartets_fp64;     /* evaluated in FP64 */
   int64_t quartets_fp32;     /* evaluated in FP32 (mixed form) */
   int64_t quartets_skipped;  /* skipped by density screening */
@@ -118,8 +122,10 @@ typedef struct {
    * density when max|D| over its Coulomb blocks times the quartet's largest
    * integral is below 10^-ifthrs, bit 2 likewise its exchange contribution
    * (INTFC1, DALTON/abacus/her2fck.F:221-222,446-466).  Dalton's default is
-   * 3.  The thread- and warp-per-quartet kernels apply it; quartets of the
-   * cooperative kernels are always digested whole (the conservative side). */
+   * 3.  The row, pack, thread- and warp-per-quartet kernels apply it, to
+   * quartets whose Dalton blocks are one working shell each; the others
+   * (blocks resolved into primitives, and all quartets of the cooperative
+   * kernels) are always digested whole, the conservative side. */
   dgf_int icedif;
   /* Range-separated exchange of CAM-type functionals (Dalton's HFXMU and
    * HFXATT, set by dftsetcam, DALTON/dft/dft_aux.F:346-351): with hfxmu != 0
@@ -216,7 +222,8 @@ typedef struct {
   int32_t kernel;           /* 0 = thread-per-quartet, 1 = cooperative team, 2 = warp teams,
                                4 = warp-per-quartet (L >= 4), 6 = warp-per-quartet with
                                FP64 tensor-core (DMMA) transforms, 8 = row kernel (a warp on
-                               bra pairs of one A shell times 32 kets),
+                               bra pairs of one A shell times 32 kets), 10 = pack kernel (a
+                               warp on one bra and several kets, DMMA transforms),
                                5 = two-electron gradient (dgf_grad2e*: quartets are the plan's,
                                primitive quartets estimated from the classes' mean primitive
                                pairs) */
@@ -297,12 +304,17 @@ int dgf_autotune(dgf_ctx *ctx, const double *dmat_device, const dgf_options *opt
 int dgf_copy_tuning(dgf_ctx *dst, const dgf_ctx *src);
 
 /* Pin the kernel of one quartet class (la lb|lc ld), as the autotuner would:
- * precision 64 or 32; variant -5 row kernel (FP64, single-primitive pairs),
+ * precision 64 or 32; variant -6 pack kernel (FP64, single-primitive pairs,
+ * spherical functions, bras with a d or f shell), -5 row kernel (FP64,
+ * single-primitive pairs),
  * -4 warp per quartet with FP64 tensor-core (DMMA) transforms, -3 warp per quartet, -2 warp team, -1
  * cooperative team, 0.. thread-kernel chunk variants.  Launches the chosen
  * kernel cannot serve (e.g. a warp kernel restricted to one primitive pair
  * per side) fall back to the default kernel.  DGF_ERR_UNSUPPORTED when the
- * variant does not exist for the class. */
+ * variant does not exist for the class.  The classes are those of the
+ * context's own pairs: in a basis with segmented contractions a pinned context
+ * runs its whole builds, gradients and batches on its contracted pairs, shards
+ * excepted. */
 int dgf_set_class_kernel(dgf_ctx *ctx, int la, int lb, int lc, int ld, int precision, int variant);
 
 /* Measurement helper (not part of the HERFCK contract): FP64 and FP32 FMA
