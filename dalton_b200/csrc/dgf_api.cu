@@ -1651,8 +1651,10 @@ static int fock_impl(dgf_ctx *c, int ndmat, const dgf_int *ifctyp, const double 
     if (outs[k].zero) DGF_CUDA_CHECK(cudaMemsetAsync(fmat_dev + (size_t)k * n2ao, 0, n2ao * 8, st));
   const int nws = c->nwshell;
   const int *d_shinfo = c->d_shinfo;
-  for (int s0 = 0; s0 < nslot_total; s0 += chunk) {
-    const int ns = std::min(chunk, nslot_total - s0);
+  for (int s0 = 0, ns = 0; s0 < nslot_total; s0 += ns) {
+    ns = std::min(chunk, nslot_total - s0);
+    // the two slots of a general density, D and D^T, are combined in one chunk
+    if (s0 + ns < nslot_total && slots[s0 + ns].op == 1) --ns;
     for (int s = 0; s < ns; ++s) {
       const SlotSpec &sp = slots[s0 + s];
       launch_work_prep(wmaps, dmat_dev + (size_t)sp.src * n2ao, c->d_D + s * n2, c->d_Ds + s * n2, sp.op,

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "dgf_internal.h"
+#include "dgf_work.h"
 
 namespace {
 
@@ -289,6 +290,11 @@ cudaError_t cudaLaunchKernel(const void *f, dim3 grid, dim3, void **args, size_t
   ++g_launches;
   const auto it = g_kernel.find(f);
   if (it == g_kernel.end()) return ret(cudaErrorInvalidDeviceFunction);
+  if (it->second.find("work_combine_kernel") != std::string::npos) {
+    const dgf::WorkMaps &m = *(const dgf::WorkMaps *)args[0];
+    for (int k = 1; k <= 2; ++k)
+      if (!live(*(const double **)args[k], m.w_elem[m.nmol] * sizeof(double))) bad(it->second, "half Fock matrices");
+  }
   if (it->second.find("jk_") != std::string::npos && it->second.find("JKArgs") != std::string::npos) {
     const dgf::JKArgs &a = *(const dgf::JKArgs *)args[0];
     const void *reads[] = {a.bra,  a.ket,  a.pp,   a.boys,  a.sph,       a.qoff,    a.blk_gab,

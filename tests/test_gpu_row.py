@@ -116,6 +116,19 @@ def test_several_densities(cuda, name):
         assert np.abs(f[k] - g).max() < 1e-15 * bs.nbf * max(1.0, np.abs(g).max())
 
 
+@pytest.mark.parametrize("ifctyp", [[13, 3, 3, 3, 3], [22, 2, 1, 11, 23, 3], [13] * 7 + [3, 3, 13]])
+def test_general_density_at_the_slot_limit(cuda, ifctyp):
+    """A general density whose two slots would be the last of one pass over the
+    quartets and the first of the next; against one build per density."""
+    bs = build_basis(molecules.water_cluster(2, seed=4), "cc-pVDZ")
+    fb = FockBuilder(bs)
+    d = np.random.default_rng(2).normal(size=(len(ifctyp), bs.nbf, bs.nbf)) * 0.1
+    f = fb.herfck(d, ifctyp)
+    for k, i in enumerate(ifctyp):
+        g = fb.herfck(d[k], i)
+        assert np.abs(f[k] - g).max() < 1e-15 * bs.nbf * max(1.0, np.abs(g).max())
+
+
 @pytest.mark.parametrize("name", ["h2o3_dz", "h2o2_aug", "c2h6_tz"])
 def test_several_densities_by_slot(cuda, name):
     """Several slots through the row kernels, one launch per slot, against the

@@ -337,3 +337,23 @@ def test_contexts_of_a_batch_stay_small(host, basis):
     assert r["batch"] == 5 + 3 * (forms - 1)  # its own five, and one of each resolved form
     assert (r["first"], r["later"]) == (7, 0)
     assert r["left"] == [0, 0] and r["bad"] == ""
+
+
+# 10 X + Y per density; a general one (X = 0) takes two of the eight slots that
+# are built at once
+MANY = [[13] * 8, [13] * 9, [3] * 5, [13, 3, 3, 3, 3], [22, 2, 1, 11, 23, 3], [13] * 7 + [3, 3, 13], [13] * 15 + [3] * 8]
+
+
+@pytest.mark.parametrize("ifctyp", MANY)
+def test_many_densities_stay_in_their_buffers(host, ifctyp):
+    """More density slots than are built at once: every combination of half
+    Fock matrices lies in their buffer."""
+    r = host(f"""
+    fb = builder("cc-pVDZ")
+    ict = {ifctyp!r}
+    d = np.zeros((len(ict), fb.nbf, fb.nbf))
+    F.fake_reset()
+    s = status(fb.herfck, d, ict, thrs=1e-4)
+    out(s=s, bad=F.fake_bad().decode())
+    """)
+    assert r == dict(s=0, bad="")
