@@ -23,7 +23,11 @@
  *     the Fortran shim maps a nonzero status to QUIT (gptrygve.F:256).
  *
  * All pointers are host pointers unless a name says _device.  A context is
- * not thread-safe; separate contexts are independent.
+ * not thread-safe; separate contexts are independent.  Calls on one context
+ * share its buffers: the caller orders them, on one stream or with a wait
+ * between streams (the host-pointer forms run on the context's own stream,
+ * which does not wait for the legacy default stream, and wait for their
+ * result).
  */
 #ifndef DGFOCK_H
 #define DGFOCK_H
