@@ -95,6 +95,19 @@ __device__ __forceinline__ double kin_1d(const double *s, int i, int j, double e
   return v;
 }
 
+// The same as 1/2 <i'|j'>, over the overlaps s[i <= I + 1][j <= J + 1]: without
+// kin_1d's difference of terms as large as the exponent, which for a tight
+// function beside a diffuse one leaves the rounding of the tight exponent.
+template <int J>
+__device__ __forceinline__ double kin_sym_1d(const double *s, int i, int j, double ea, double eb) {
+  constexpr int ST = J + 2;
+  double v = 2.0 * ea * eb * s[(i + 1) * ST + j + 1];
+  if (j > 0) v -= ea * j * s[(i + 1) * ST + j - 1];
+  if (i > 0) v -= eb * i * s[(i - 1) * ST + j + 1];
+  if (i > 0 && j > 0) v += 0.5 * i * j * s[(i - 1) * ST + j - 1];
+  return v;
+}
+
 template <int LA, int LB, bool SPH>
 __global__ void __launch_bounds__(kOneBlock) oneint_kernel(const OneArgs a) {
   constexpr int NA = ncart(LA), NB = ncart(LB), LAB = LA + LB, NH = n3(LAB);
@@ -114,18 +127,20 @@ __global__ void __launch_bounds__(kOneBlock) oneint_kernel(const OneArgs a) {
       const PrimPair P = load_prim<true>(pp + m);
       const double eb = P.p - P.ea, h = 0.5 / P.p, kab = P.K * P.p * kInvR2Pi52;
       {
-        double sx[(LA + 1) * (LB + 3)], sy[(LA + 1) * (LB + 3)], sz[(LA + 1) * (LB + 3)];
-        overlap_1d<LA, LB + 2>(h, P.PAx, P.PBx, sx);
-        overlap_1d<LA, LB + 2>(h, P.PAy, P.PBy, sy);
-        overlap_1d<LA, LB + 2>(h, P.PAz, P.PBz, sz);
+        constexpr int ST = LB + 2;
+        double sx[(LA + 2) * ST], sy[(LA + 2) * ST], sz[(LA + 2) * ST];
+        overlap_1d<LA + 1, LB + 1>(h, P.PAx, P.PBx, sx);
+        overlap_1d<LA + 1, LB + 1>(h, P.PAy, P.PBy, sy);
+        overlap_1d<LA + 1, LB + 1>(h, P.PAz, P.PBz, sz);
         const double r = kPi / P.p, s0 = r * sqrt(r) * kab;
         comp_loop<ROLL, NA, NB>([&](auto ia, auto ib) {
             const int ax = cart_x(LA, ia), ay = cart_y(LA, ia), az = cart_z(LA, ia);
             const int bx = cart_x(LB, ib), by = cart_y(LB, ib), bz = cart_z(LB, ib);
-            const double x = sx[ax * (LB + 3) + bx], y = sy[ay * (LB + 3) + by], z = sz[az * (LB + 3) + bz];
+            const double x = sx[ax * ST + bx], y = sy[ay * ST + by], z = sz[az * ST + bz];
             S[ia * NB + ib] += s0 * (x * y * z);
-            T[ia * NB + ib] += s0 * (kin_1d<LB>(sx, ax, bx, eb) * y * z + x * kin_1d<LB>(sy, ay, by, eb) * z +
-                                     x * y * kin_1d<LB>(sz, az, bz, eb));
+            T[ia * NB + ib] += s0 * (kin_sym_1d<LB>(sx, ax, bx, P.ea, eb) * y * z +
+                                     x * kin_sym_1d<LB>(sy, ay, by, P.ea, eb) * z +
+                                     x * y * kin_sym_1d<LB>(sz, az, bz, P.ea, eb));
           });
       }
       if (a.V) {

@@ -55,6 +55,31 @@ def test_one_electron(cuda, orc, name):
         assert np.abs(g - ref).max() < 1e-14 * bs.nbf * max(1.0, np.abs(ref).max())
 
 
+@pytest.mark.parametrize("basis", ["cc-pVDZ", "6-31G*", "STO-3G"])
+def test_kinetic_energy_of_s_functions(cuda, basis):
+    """T between s functions against its closed form, a b / p (3 - 2 mu R^2) S,
+    in extended precision: some fifteen roundings of each primitive's term
+    (2e-15 of the terms' sum), also where a tight function meets a diffuse
+    one."""
+    bs = build_basis(molecules.water_dalton_test(), basis)
+    ld = np.longdouble
+    fun = []
+    for i in np.nonzero(np.asarray(bs.block_l) == 0)[0]:
+        c = np.asarray(bs.block_coefs(i)).astype(ld)
+        x = bs.molecule.coords[int(bs.block_atom[i])].astype(ld)
+        fun += [(int(bs.block_ao_offset[i]) + k, np.asarray(bs.block_exps(i)).astype(ld), c[:, k], x)
+                for k in range(c.shape[1])]
+    T = FockBuilder(bs).oneint()[1]
+    pi = ld("3.14159265358979323846264338327950288")
+    for m, a, ca, xa in fun:
+        for n, b, cb, xb in fun:
+            p = a[:, None] + b[None, :]
+            mu = a[:, None] * b[None, :] / p
+            r2 = ((xa - xb) ** 2).sum()
+            t = ca[:, None] * cb[None, :] * np.exp(-mu * r2) * (pi / p) ** ld(1.5) * mu * (3 - 2 * mu * r2)
+            assert abs(float(T[m, n] - t.sum())) < 2e-15 * float(np.abs(t).sum()), (m, n)
+
+
 @pytest.mark.parametrize("sph", [True, False])
 def test_one_electron_of_distant_shells(cuda, orc, sph):
     """Two atoms 10.3 bohr apart: the overlap distributions of their f shells
